@@ -719,6 +719,13 @@ static bool schedule_rstage(const std::vector<const PendingGate *> &gates, const
     return true;
 }
 
+// Whether every gate's lanes in the tile fit one fused block.
+static bool narrow_gates(const std::vector<const PendingGate *> &gates, unsigned long long S) {
+    for (const PendingGate *g : gates)
+        if (__builtin_popcountll(gate_qmask(*g) & S) > kTcBlockLanes) return false;
+    return true;
+}
+
 static void run_tstage(Device &d, States *s, const TileLanes &tl,
                        const std::vector<const PendingGate *> &gates) {
     const int n = s->n_lanes;
@@ -788,7 +795,8 @@ static void run_stage(Device &d, States *s, unsigned long long S,
     const int m = (int)tl.lanes.size();
     // Valid shapes: 32..512 threads (256 with 5 register lanes), 3..5
     // register lanes (complex128 at most 4).
-    if (d.tensor_blocks && s->prec == kFP32 && (m == 12 || m == 13) && n >= m) {
+    if (d.tensor_blocks && s->prec == kFP32 && (m == 12 || m == 13) && n >= m &&
+        narrow_gates(gates, S)) {
         run_tstage(d, s, tl, gates);
         return;
     }
@@ -888,7 +896,7 @@ static void flush_lookahead(Device &d, States *s, std::vector<const PendingGate 
     const int n = s->n_lanes;
     for (int done = 0; !remaining.empty() && done < max_stages; ++done) {
         const unsigned long long q0 = gate_qmask(*remaining[0]);
-        if (__builtin_popcountll(q0 | base) > M) {
+        if (__builtin_popcountll(q0 | base) > M || __builtin_popcountll(q0) > kTcBlockLanes) {
             run_single_gate(d, s, *remaining[0]);
             remaining.erase(remaining.begin());
             continue;

@@ -34,6 +34,10 @@ TileLanes tile_lanes_of(unsigned long long S, int n);
 // on its one lane in the tile (or a per-tile scalar).
 bool cross_gate(const PendingGate &g, unsigned long long S);
 
+// Lanes of a fused block.  A gate on more lanes of its tile fits no block: it
+// runs as a pass of its own.
+constexpr int kTcBlockLanes = 5;
+
 // Gates (in order) a stage on lane set S takes, commutation-safe; at most
 // `limit` scanned and `max_take` taken.  With `cross`, cross gates count as
 // fitting S.  Returns the count; fills take/keep when given.

@@ -46,7 +46,8 @@ bool cross_gate(const PendingGate &g, unsigned long long S) {
 }
 
 // Gates of `gates` (in order) that a stage on lane set S takes: a gate is
-// taken when its lanes lie in S (or, with `cross`, it is a cross gate) and
+// taken when its lanes, at most the five of a fused block, lie in S (or, with
+// `cross`, it is a cross gate) and
 // no earlier gate that was left out shares a lane with it (so it commutes
 // with everything left out before it).  At most `limit` gates are scanned
 // and `max_take` taken; returns the count.
@@ -63,7 +64,8 @@ int stage_take(const std::vector<const PendingGate *> &gates, unsigned long long
             continue;
         }
         const unsigned long long q = gate_qmask(*g);
-        const bool fits = !(q & ~S) || (cross && cross_gate(*g, S));
+        const bool fits = (!(q & ~S) && __builtin_popcountll(q) <= kTcBlockLanes) ||
+                          (cross && cross_gate(*g, S));
         if ((q & blocked) || !fits || count >= max_take) {
             blocked |= q;
             if (keep) keep->push_back(g);
@@ -86,7 +88,8 @@ static int take_count(const std::vector<unsigned long long> &q, const std::vecto
     int count = 0;
     for (size_t i = 0; i < q.size(); ++i) {
         const unsigned long long g = q[i];
-        const bool fits = !(g & ~S) || (cross && xd[i] && __builtin_popcountll(g & S) <= 1);
+        const bool fits = (!(g & ~S) && __builtin_popcountll(g) <= kTcBlockLanes) ||
+                          (cross && xd[i] && (g & ~S) && __builtin_popcountll(g & S) <= 1);
         if ((g & blocked) || !fits || count >= max_take) {
             blocked |= g;
             if (!cross && (blocked & S) == S) break;
