@@ -42,10 +42,10 @@ CANDIDATES = {
                  (12, 5, 0, 0, 0), (13, 4, 0, 0, 0), (13, 5, 0, 0, 0), (12, 4, 130, 0, 0),
                  (11, 4, 130, 0, 0), (12, 5, 0, 1, 0), (12, 5, 0, 1, 1), (13, 5, 0, 1, 0)],
     np.float64: [(10, 4, 0, 0, 0), (11, 4, 0, 0, 0), (12, 4, 0, 0, 0), (13, 4, 0, 0, 0),
-                 (11, 3, 0, 0, 0), (12, 3, 0, 0, 0)],
+                 (11, 3, 0, 0, 0), (12, 3, 0, 0, 0), (12, 3, 0, 1, 0)],
 }
 # bumped whenever the kernels change in a way that can reorder the candidates
-_VERSION = 'v4'
+_VERSION = 'v5'
 
 
 def _norm(c):
@@ -110,7 +110,7 @@ def _time_candidates(n_lanes, dtype, ops, repeats, cands):
     results = []
     for cand in cands:
         tile, rl, budget, tensor, prefetch = _norm(cand)
-        if tile > n_lanes or (tensor and dtype == np.float64):
+        if tile > n_lanes:
             continue
         nat.set_fusion_params(prec, tile, rl, budget)
         nat.set_tensor_blocks(tensor)

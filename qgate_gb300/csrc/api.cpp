@@ -726,19 +726,38 @@ static bool narrow_gates(const std::vector<const PendingGate *> &gates, unsigned
     return true;
 }
 
+// Whether the diagonal gates can run as fixed-point phases (entries of modulus
+// at most 1).
+static bool bounded_phases(const std::vector<const PendingGate *> &gates) {
+    for (const PendingGate *g : gates)
+        if (g->diag && !(std::hypot(g->m.v[0], g->m.v[1]) < 1. + 1e-9 &&
+                         std::hypot(g->m.v[6], g->m.v[7]) < 1. + 1e-9))
+            return false;
+    return true;
+}
+
+// Digits can only be cut from finite matrices; a stage with another one runs
+// on the CUDA cores.
+static bool finite_gates(const std::vector<const PendingGate *> &gates) {
+    for (const PendingGate *g : gates)
+        for (double v : g->m.v)
+            if (!(std::fabs(v) < 1e100)) return false;
+    return true;
+}
+
 static void run_tstage(Device &d, States *s, const TileLanes &tl,
                        const std::vector<const PendingGate *> &gates) {
     const int n = s->n_lanes;
-    const TcOps ops = tc_ops(tc_blocks(gates, tl), true);
+    const TcOps ops = tc_ops(tc_blocks(gates, tl), s->prec == kFP32 || bounded_phases(gates));
     if (!d.h_bring) {
         QG_CUDA(cudaMallocHost(&d.h_bring, Device::kBRingBytes));
         QG_CUDA(cudaMalloc(&d.d_bring, Device::kBRingBytes));
         d.bring_off = 0;
     }
     for (size_t b0 = 0; b0 < ops.size();) {
-        const int nb = tc_ops_per_launch(ops, b0);
+        const int nb = tc_ops_per_launch(ops, b0, s->prec);
         size_t bytes = 0;
-        for (int b = 0; b < nb; ++b) bytes += tc_op_bytes(ops[b0 + b]);
+        for (int b = 0; b < nb; ++b) bytes += tc_op_bytes(ops[b0 + b], s->prec);
         unsigned char *hb, *db;
         if (d.capturing) {
             // operands a captured graph re-reads: chunks owned by the circuit
@@ -766,10 +785,15 @@ static void run_tstage(Device &d, States *s, const TileLanes &tl,
             d.bring_off += bytes;
         }
         static TcStageDesc desc;
-        tc_plan_launch(tl, n, ops, b0, nb, desc, hb);
+        tc_plan_launch(tl, n, ops, b0, nb, desc, hb, s->prec);
         desc.bmats = db;
         QG_CUDA(cudaMemcpyAsync(db, hb, bytes, cudaMemcpyHostToDevice, d.stream));
-        timed(d, "tstage", [&] { launch_tstage(s->d, desc, d.stream, d.pipelined); });
+        timed(d, "tstage", [&] {
+            if (s->prec == kFP64)
+                launch_dstage(s->d, desc, d.stream);
+            else
+                launch_tstage(s->d, desc, d.stream, d.pipelined);
+        });
         d.n_passes += 1;
         d.n_bytes += 2 * ((long long)1 << n) * (long long)complex_size(s->prec);
         b0 += nb;
@@ -795,8 +819,8 @@ static void run_stage(Device &d, States *s, unsigned long long S,
     const int m = (int)tl.lanes.size();
     // Valid shapes: 32..512 threads (256 with 5 register lanes), 3..5
     // register lanes (complex128 at most 4).
-    if (d.tensor_blocks && s->prec == kFP32 && (m == 12 || m == 13) && n >= m &&
-        narrow_gates(gates, S)) {
+    if (d.tensor_blocks && (m == 12 || (m == 13 && s->prec == kFP32)) && n >= m &&
+        narrow_gates(gates, S) && (s->prec == kFP32 || finite_gates(gates))) {
         run_tstage(d, s, tl, gates);
         return;
     }
@@ -903,9 +927,10 @@ static void flush_lookahead(Device &d, States *s, std::vector<const PendingGate 
         }
         // cross gates (diagonal gates with at most one lane in the tile) run
         // in any stage as per-tile phases
-        unsigned long long S = plan_stage_lanes(remaining, base, M, true, kMaxTensorStageGates);
+        const bool cross = s->prec == kFP32;
+        unsigned long long S = plan_stage_lanes(remaining, base, M, cross, kMaxTensorStageGates);
         std::vector<const PendingGate *> chosen, deferred;
-        stage_take(remaining, S, remaining.size(), &chosen, &deferred, true, kMaxTensorStageGates);
+        stage_take(remaining, S, remaining.size(), &chosen, &deferred, cross, kMaxTensorStageGates);
         if (chosen.size() == 1) {
             run_single_gate(d, s, *chosen[0]);
         } else {
@@ -916,13 +941,19 @@ static void flush_lookahead(Device &d, States *s, std::vector<const PendingGate 
     }
 }
 
+// The lowest lanes, in every tile so that it is made of 128-byte runs.
+static unsigned long long stage_low_lanes(const States *s) {
+    return (1ULL << std::min(s->n_lanes, s->prec == kFP32 ? 4 : 3)) - 1;
+}
+
 // Whether a states object's pending gates go to the lookahead planner of
 // tensor-core stages, and its tile size M and always-present lanes `base`.
 static bool lookahead_params(const Device &d, const States *s, int &M, unsigned long long &base) {
     const int n = s->n_lanes;
     M = std::min(d.tile_lanes[s->prec], kMaxTileLanes);
-    if (!(d.tensor_blocks && s->prec == kFP32 && (M == 12 || M == 13) && n > M)) return false;
-    base = (1ULL << std::min(n, 4)) - 1;
+    const bool tile = M == 12 || (M == 13 && s->prec == kFP32);
+    if (!(d.tensor_blocks && tile && n > M)) return false;
+    base = stage_low_lanes(s);
     return true;
 }
 
@@ -1020,12 +1051,13 @@ static void flush(States *s) {
     if (s->prec == kFP64 && M > 13) M = 13;
     const int budget = d.cost_budget[s->prec];
     const int rl = d.reg_lanes[s->prec];
-    const int low = std::min(n, s->prec == kFP32 ? 4 : 3);
     const unsigned long long all = n >= 64 ? ~0ULL : ((1ULL << n) - 1);
     if (n <= M) M = n;
-    const unsigned long long base = (n <= M) ? all : ((1ULL << low) - 1);
-    if (d.tensor_blocks && s->prec == kFP32 && (M == 12 || M == 13) && n > M) {
-        flush_lookahead(d, s, remaining, base, M);
+    const unsigned long long base = (n <= M) ? all : stage_low_lanes(s);
+    unsigned long long tbase;
+    int tM;
+    if (lookahead_params(d, s, tM, tbase)) {
+        flush_lookahead(d, s, remaining, tbase, tM);
         s->pending.clear();
         return;
     }
@@ -2044,7 +2076,7 @@ int qg_tensor_stage_status(int reset, int *status) {
     Device &d = dev();
     flush_all();
     QG_CUDA(cudaStreamSynchronize(d.stream));
-    *status = tstage_status(reset != 0);
+    *status = tstage_status(reset != 0) | (dstage_status(reset != 0) << 8);
     QG_END
 }
 

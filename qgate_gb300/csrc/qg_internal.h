@@ -191,12 +191,23 @@ struct TcStageDesc {
     unsigned ops_bytes;
     unsigned op_off[kMaxTcBlocks];        // byte offset of op b's operands
     unsigned char op_kind[kMaxTcBlocks];  // 0: dense block, 1: phase table, 2: cross
+    short op_exp[kMaxTcBlocks];           // complex128: op b's matrix is its digits * 2^op_exp
     const unsigned char *bmats;
     SetSlots sets[kMaxTcBlocks + 2];
 };
 // two_per_row: the 12-lane variant with two threads per tile row (twice the
 // warps per SM, half the registers per thread).
 void launch_tstage(void *state, const TcStageDesc &d, cudaStream_t stream, bool two_per_row);
+// The complex128 form (dstage.cu): 12-lane tiles, dense and phase ops; bmats
+// holds phase tables (tc_phase_table) and each block's digit slices: kDigitOpBytes as 8 chunks (half h, K-step ks at
+// 4 h + ks) of 160 rows x 16 FP16 values, row 32 (j - 1) + c of a chunk being
+// column 32 h + c of digit slice j; value (row, k) at byte (k / 8) * 2560 +
+// row / 8 * 128 + row % 8 * 16 + k % 8 * 2.
+constexpr int kDigits = 5;
+constexpr unsigned kDigitChunkBytes = 160u * 16u * 2u;
+constexpr unsigned kDigitOpBytes = 8u * kDigitChunkBytes;
+void launch_dstage(void *state, const TcStageDesc &d, cudaStream_t stream);
+int dstage_status(bool reset);
 // Status word of the tensor stage kernels (nonzero: a bounded wait gave up).
 int tstage_status(bool reset);
 

@@ -81,19 +81,20 @@ struct TcOp {
 typedef std::vector<TcOp> TcOps;
 TcOps tc_ops(const TcBlocks &blocks, bool phases);
 inline bool tc_dense(const TcOp &op) { return !op.phase && !op.cross; }
-// Operand bytes of an op: 16 KB for a dense op (Bh, Bl), 8 bytes per entry of
+// Operand bytes of an op (complex64; complex128: kDigitOpBytes for a dense op,
+// 16 bytes per entry of a phase table): 16 KB for a dense op (Bh, Bl), 8 bytes per entry of
 // a phase table (2^lanes complex64 phases), a header and 32 bytes per gate
 // for a cross op.
-size_t tc_op_bytes(const TcOp &op);
+size_t tc_op_bytes(const TcOp &op, int prec = kFP32);
 // How many ops from ops[b0] one launch holds (their operands and slot tables
 // in the shared memory a tensor-stage launch leaves for them).
-int tc_ops_per_launch(const TcOps &ops, size_t b0);
+int tc_ops_per_launch(const TcOps &ops, size_t b0, int prec = kFP32);
 
 // Host plan of one tensor-stage launch over ops [b0, b0 + nb): the
 // descriptor (all but the operand pointer) and the ops' operands in `buf`
 // (dense ops first, then the phase tables; desc.ops_bytes in all).
 void tc_plan_launch(const TileLanes &tl, int n, const TcOps &ops, size_t b0, int nb,
-                    TcStageDesc &desc, unsigned char *buf);
+                    TcStageDesc &desc, unsigned char *buf, int prec = kFP32);
 
 // Whether complex64 stages run on the tensor cores (the gate queue's setting).
 bool tensor_stages_enabled();

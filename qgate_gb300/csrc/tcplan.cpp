@@ -300,6 +300,60 @@ static void tc_operand(const std::complex<double> *U, unsigned short *bh, unsign
         }
 }
 
+// Digit operand of a 32x32 complex block U for a complex128 stage: B as in
+// tc_operand, scaled by 2^-e so that its rows have norm at most 1 (e is
+// returned: 0 for a unitary), each entry cut into kDigits balanced radix-2^10
+// digits, b1 = rint(x 2^10) and every next one rint of 2^10 times the rest
+// (exact in FP64; the last to quarters), in the chunks described at
+// kDigitOpBytes.
+static int tc_operand_digits(const std::complex<double> *U, unsigned short *out) {
+    double norm2 = 0.;
+    for (int o = 0; o < 32; ++o) {
+        double row = 0.;
+        for (int i = 0; i < 32; ++i) row += std::norm(U[o * 32 + i]);
+        norm2 = std::max(norm2, row);
+    }
+    // (a unitary's rows miss 1 by rounding only)
+    int e = 0;
+    if (norm2 > 0.) {
+        std::frexp(std::sqrt(norm2) * (1. - 1e-9), &e);
+    }
+    const double scale = std::ldexp(1., 10 - e);
+    // b in FP16: |b| <= 1024, exact (the table's index is 4 b + 4096).  The
+    // last digit keeps quarters, which FP16 holds up to 512: two more bits.
+    static const std::vector<unsigned short> f16 = [] {
+        std::vector<unsigned short> t(8193);
+        for (int b = -4096; b <= 4096; ++b) t[b + 4096] = f16_bits(0.25f * (float)b);
+        return t;
+    }();
+    for (int o = 0; o < 32; ++o)
+        for (int i = 0; i < 32; ++i)
+            for (int part = 0; part < 2; ++part) {
+                // (row, column) of D = A B are (k, n): re at (2i, 2o) and
+                // (2i + 1, 2o + 1), im at (2i, 2o + 1), -im at (2i + 1, 2o)
+                double x = (part ? U[o * 32 + i].imag() : U[o * 32 + i].real()) * scale;
+                const size_t at = (size_t)(4 * (o >> 4) + (i >> 3)) * (kDigitChunkBytes / 2) +
+                                  (i % 8 / 4) * 1280 + (2 * o & 31) / 8 * 64 + (2 * o & 7) * 8 +
+                                  2 * (i & 3);
+                unsigned short *p = out + at;
+                for (int j = 0; j < kDigits; ++j, p += 256) {
+                    // rint(x) for |x| <= 1024 by the 1.5 * 2^52 addition
+                    // (to quarters: 1.5 * 2^50)
+                    const double c = j + 1 < kDigits ? 6755399441055744. : 1688849860263936.;
+                    const double b = (x + c) - c;
+                    x = (x - b) * 1024.;
+                    const int v = (int)(4. * b);
+                    if (part == 0) {
+                        p[0] = p[9] = f16[4096 + v];
+                    } else {
+                        p[8] = f16[4096 + v];
+                        p[1] = f16[4096 - v];
+                    }
+                }
+            }
+    return e;
+}
+
 // Bias compensation for the tensor core's accumulator.  The FP32 accumulator
 // of tcgen05.mma rounds toward zero at every MMA, so each output shrinks in
 // magnitude by half an ulp per rounding on average; the kernel orders the
@@ -506,7 +560,8 @@ static unsigned tc_fill_lanes(unsigned lanes, const TcLayout &src, int m) {
 // per instruction, as the load layout's loads are.  (Positions 0 and 1 alone,
 // eight whole 32-byte sectors per instruction, measured slower than the trip
 // through the natural tile.)
-constexpr unsigned kDirectLow = 15u;
+// complex128: positions 0..2 (eight amplitudes) make the 128-byte line.
+static unsigned tc_direct_low(int prec) { return prec == kFP64 ? 7u : 15u; }
 
 // tc_fill_lanes that never adds the positions in `avoid`.
 static unsigned tc_fill_lanes_avoiding(unsigned lanes, const TcLayout &src, int m,
@@ -553,6 +608,17 @@ static int tc_store_cost8(const SetSlots &ss) {
     return cost;
 }
 
+// Wavefronts of one warp-wide 16-byte store (four quarter warps).
+static int tc_store_cost16(const SetSlots &ss) {
+    int cost = 0;
+    for (int h = 0; h < 4; ++h) {
+        int cnt[8] = {0}, mx = 0;
+        for (int i = 0; i < 8; ++i) mx = std::max(mx, ++cnt[ss.lo[8 * h + i] & 7]);
+        cost += mx;
+    }
+    return cost;
+}
+
 // ---------------------------------------------------------------- stage ops
 
 TcOps tc_ops(const TcBlocks &blocks, bool phases) {
@@ -589,7 +655,9 @@ TcOps tc_ops(const TcBlocks &blocks, bool phases) {
     return out;
 }
 
-size_t tc_op_bytes(const TcOp &op) {
+size_t tc_op_bytes(const TcOp &op, int prec) {
+    if (prec == kFP64)
+        return op.phase ? (size_t)16 << __builtin_popcount(op.lanes) : (size_t)kDigitOpBytes;
     if (op.cross) return sizeof(TcCrossHdr) + sizeof(TcCrossRec) * op.gates.size();
     return op.phase ? (size_t)8 << __builtin_popcount(op.lanes) : (size_t)2 * 64 * 64 * 2;
 }
@@ -601,7 +669,9 @@ size_t tc_op_bytes(const TcOp &op) {
 // natural-tile slot tables.
 constexpr size_t kTcOpsBudget = 227 * 1024 - 2048 - 128 * 1024 - 2 * sizeof(SetSlots);
 
-int tc_ops_per_launch(const TcOps &ops, size_t b0) {
+int tc_ops_per_launch(const TcOps &ops, size_t b0, int prec) {
+    // complex128 launches stream their operands from L2
+    if (prec == kFP64) return (int)std::min(ops.size() - b0, (size_t)kMaxTcBlocks);
     size_t used = 0;
     int nb = 0;
     while (b0 + nb < ops.size() && nb < kMaxTcBlocks) {
@@ -617,8 +687,10 @@ int tc_ops_per_launch(const TcOps &ops, size_t b0) {
 // the product of the op's diagonal gates' entries at that assignment of
 // their lanes (m00 or m11 of a gate whose controls are all set, else 1),
 // computed in FP64 and rounded to complex64.
+// complex128 tables hold four integers per entry: each part x as rint(x 2^30)
+// and rint of 2^32 times the rest, the real part first.
 static void tc_phase_table(const TcOp &op, const TileLanes &tl, const std::vector<int> &order,
-                           float *table) {
+                           unsigned char *out, int prec) {
     typedef std::complex<double> cd;
     const int u = (int)order.size();
     int bit_of[64];
@@ -633,8 +705,19 @@ static void tc_phase_table(const TcOp &op, const TileLanes &tl, const std::vecto
             ph *= (idx >> bit_of[tl.local_of[g->target]] & 1u) ? cd(g->m.v[6], g->m.v[7])
                                                                : cd(g->m.v[0], g->m.v[1]);
         }
-        table[2 * idx] = (float)ph.real();
-        table[2 * idx + 1] = (float)ph.imag();
+        const double part[2] = {ph.real(), ph.imag()};
+        if (prec == kFP64) {
+            int e[4];
+            for (int p = 0; p < 2; ++p) {
+                const double x = part[p] * 0x1p30, h = std::nearbyint(x);
+                e[2 * p] = (int)h;
+                e[2 * p + 1] = (int)std::min(std::nearbyint((x - h) * 0x1p32), 2147483647.);
+            }
+            memcpy(out + 16 * (size_t)idx, e, sizeof(e));
+            continue;
+        }
+        const float f[2] = {(float)part[0], (float)part[1]};
+        memcpy(out + 8 * (size_t)idx, f, sizeof(f));
     }
 }
 
@@ -642,7 +725,7 @@ static void tc_phase_table(const TcOp &op, const TileLanes &tl, const std::vecto
 // `tl` -> the descriptor (all but the operand pointer) and the ops' operands
 // in `buf`.
 static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops, size_t b0,
-                                   int nb, TcStageDesc &desc, unsigned char *buf);
+                                   int nb, TcStageDesc &desc, unsigned char *buf, int prec);
 
 // Header and records of a cross op in the layout `lay` it runs in: one record
 // per gate (its two phases as angles), by the tile position of its one lane
@@ -684,7 +767,8 @@ static void tc_cross_records(const TcOp &op, const TileLanes &tl, const TcLayout
 }
 
 void tc_plan_launch(const TileLanes &tl, int n, const TcOps &ops, size_t b0, int nb,
-                    TcStageDesc &desc, unsigned char *buf) {
+                    TcStageDesc &desc, unsigned char *buf, int prec) {
+    const unsigned kDirectLow = tc_direct_low(prec);
     // The launch's ops in an order that ends with a dense op leaving tile
     // positions 0..3 to the rows (its rows then go straight to the state):
     // a dense op moves to the end when it shares no lane with any op after
@@ -706,11 +790,12 @@ void tc_plan_launch(const TileLanes &tl, int n, const TcOps &ops, size_t b0, int
             }
         }
     }
-    tc_plan_launch_ordered(tl, n, slice, 0, nb, desc, buf);
+    tc_plan_launch_ordered(tl, n, slice, 0, nb, desc, buf, prec);
 }
 
 static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops, size_t b0,
-                                   int nb, TcStageDesc &desc, unsigned char *buf) {
+                                   int nb, TcStageDesc &desc, unsigned char *buf, int prec) {
+    const unsigned kDirectLow = tc_direct_low(prec);
     const int m = (int)tl.lanes.size();
     const int t = m - 5;
     memset(&desc, 0, sizeof(desc));
@@ -729,7 +814,7 @@ static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops,
             for (int b = 0; b < nb; ++b)
                 if (kind(ops[b0 + b]) == pass) {
                     desc.op_off[b] = off;
-                    off += (unsigned)tc_op_bytes(ops[b0 + b]);
+                    off += (unsigned)tc_op_bytes(ops[b0 + b], prec);
                 }
         desc.ops_bytes = off;
     }
@@ -784,7 +869,7 @@ static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops,
         desc.dep_hi[j] = off;
     }
     for (int k = 0; k < 5; ++k) desc.in_e[k] = desc.dep_hi[1 << k];
-    desc.sets[nb + 1] = tc_slots(cur, t, [&](unsigned ti) { return host_swz(ti, kFP32); });
+    desc.sets[nb + 1] = tc_slots(cur, t, [&](unsigned ti) { return host_swz(ti, prec); });
     std::complex<double> U[1024];
     for (int b = 0; b < nb; ++b) {
         const TcOp &op = ops[b0 + b];
@@ -809,7 +894,7 @@ static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops,
                     if (ti >> order[k] & 1u) idx |= 1u << k;
                 return idx;
             });
-            tc_phase_table(op, tl, order, (float *)(buf + desc.op_off[b]));
+            tc_phase_table(op, tl, order, buf + desc.op_off[b], prec);
             continue;
         }
         // The last dense op stores its rows straight to the state when its
@@ -858,8 +943,9 @@ static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops,
                     TcLayout c = keep;
                     std::swap(c.rows[3], c.rows[x]);
                     std::swap(c.rows[4], c.rows[y == 3 ? x : y]);
-                    const int cost = tc_store_cost8(
-                        tc_slots(c, t, [&](unsigned ti) { return host_swz(ti, kFP32); }));
+                    const SetSlots nat =
+                        tc_slots(c, t, [&](unsigned ti) { return host_swz(ti, prec); });
+                    const int cost = prec == kFP64 ? tc_store_cost16(nat) : tc_store_cost8(nat);
                     if (cost < best) {
                         best = cost;
                         lay = c;
@@ -869,12 +955,16 @@ static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops,
         desc.op_kind[b] = 0;
         desc.sets[b] = tc_slots(cur, t, [&](unsigned ti) { return tc_operand_slot(lay, ti); });
         tc_block_matrix(op.gates, tl, lay, U);
-        tc_compensate(U);
         unsigned short *o = (unsigned short *)(buf + desc.op_off[b]);
-        tc_operand(U, o, o + 64 * 64);
+        if (prec == kFP64) {
+            desc.op_exp[b] = (short)tc_operand_digits(U, o);
+        } else {
+            tc_compensate(U);
+            tc_operand(U, o, o + 64 * 64);
+        }
         cur = lay;
     }
-    desc.sets[nb] = tc_slots(cur, t, [&](unsigned ti) { return host_swz(ti, kFP32); });
+    desc.sets[nb] = tc_slots(cur, t, [&](unsigned ti) { return host_swz(ti, prec); });
     desc.direct_out = direct_out ? 1 : 0;
     for (int b = 0; b < 8; ++b) desc.out_row_lane[b] = b < t ? tl.lanes[cur.rows[b]] : 0;
     for (int k = 0; k < 5; ++k) desc.out_e[k] = 1LL << tl.lanes[cur.amps[k]];

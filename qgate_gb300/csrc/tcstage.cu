@@ -45,6 +45,7 @@
 #include "qg_device.cuh"
 #include "qg_internal.h"
 #include "qg_regstage.cuh"
+#include "qg_tc.cuh"
 
 namespace qg {
 
@@ -52,42 +53,7 @@ __device__ unsigned g_tc_status;
 
 namespace {
 
-
-// Shared-memory matrix descriptor: start address, leading-dimension byte
-// offset (between core matrices along K; unused by swizzled K-major
-// layouts), stride-dimension byte offset (between 8-row groups), descriptor
-// version 1, layout type (0 = no swizzle, 2 = 128-byte swizzle).
-__device__ __forceinline__ uint64_t smem_desc(unsigned saddr, unsigned lbo, unsigned sbo,
-                                              unsigned layout = 0) {
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) |
-           ((uint64_t)(sbo >> 4) << 32) | (1ull << 46) | ((uint64_t)layout << 61);
-}
-
-// Instruction descriptor of kind::f16: D = F32, A = B = F16, both K-major,
-// N = 64, M = 128.
-constexpr unsigned kIdescF16 = (1u << 4) | (0u << 7) | (0u << 10) | ((64u >> 3) << 17) |
-                               ((128u >> 4) << 24);
-
-__device__ __forceinline__ void mma_f16(unsigned dtmem, uint64_t a, uint64_t b, unsigned acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %4, p;\n\t}\n" ::"r"(dtmem),
-        "l"(a), "l"(b), "r"(acc), "r"(kIdescF16)
-        : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(unsigned bar) {
-    asm volatile(
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
-        : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-}
+constexpr unsigned kIdescF16 = idesc_f16(128, 64);
 
 __device__ __forceinline__ void tmem_ld_x64(unsigned taddr, unsigned (&u)[64]) {
     asm volatile(
@@ -113,10 +79,6 @@ __device__ __forceinline__ void tmem_ld_x32(unsigned taddr, unsigned (&u)[32]) {
         : "r"(taddr));
 }
 
-__device__ __forceinline__ void tmem_wait_ld() {
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-}
-
 // (hi, lo) FP16 split of a complex amplitude (x, y): hi = f16x2(x, y)
 // rounded to nearest, lo = f16x2 of the residuals.
 __device__ __forceinline__ void split_f16x2(float x, float y, unsigned &hi, unsigned &lo) {
@@ -130,16 +92,6 @@ __device__ __forceinline__ void split_f16x2(float x, float y, unsigned &hi, unsi
         "cvt.rn.f16x2.f32 %1, hy, hx;\n\t}\n"
         : "=r"(hi), "=r"(lo)
         : "f"(x), "f"(y));
-}
-
-// Bit in which the Gray codes of i - 1 and i differ (ctz(i)), at compile
-// time once the loops are unrolled.
-__host__ __device__ constexpr int gray_bit(int i) {
-    return (i & 1) ? 0 : (i & 2) ? 1 : (i & 4) ? 2 : (i & 8) ? 3 : 4;
-}
-// Inverse Gray code of j (5 bits).
-__host__ __device__ constexpr int gray_index(int j) {
-    return j ^ (j >> 1) ^ (j >> 2) ^ (j >> 3) ^ (j >> 4);
 }
 
 // Visits the 2^NB registers of a thread in Gray-code order: f(j, p) with
@@ -163,10 +115,6 @@ __device__ __forceinline__ void gray_walk(P *base, const long long (&e)[5], F f)
 constexpr float kScale = 4096.f, kUnscale = 1.f / 4096.f;
 
 }  // namespace
-
-__device__ __forceinline__ void group_sync(unsigned id, unsigned threads) {
-    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
-}
 
 // Persistent kernel, one CTA per SM.  The CTA holds every block operand of
 // the stage in shared memory (loaded once) and G independent tile groups;
@@ -421,14 +369,14 @@ k_tstage(float2 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tile
                             const uint64_t dal = smem_desc(al + aoff, 16, 1024, 2);
                             const uint64_t dbh = smem_desc(bh + boff, 1024, 128);
                             const uint64_t dbl = smem_desc(bl + boff, 1024, 128);
-                            mma_f16(dcol, dah, dbl, ks > 0 ? 1u : 0u);
-                            mma_f16(dcol, dal, dbh, 1u);
+                            mma_f16(dcol, dah, dbl, ks > 0 ? 1u : 0u, kIdescF16);
+                            mma_f16(dcol, dal, dbh, 1u, kIdescF16);
                         }
 #pragma unroll
                         for (int ks = 0; ks < 4; ++ks) {
                             const unsigned aoff = 16384u * mt + 32u * ks, boff = 2048u * ks;
                             mma_f16(dcol, smem_desc(ah + aoff, 16, 1024, 2),
-                                    smem_desc(bh + boff, 1024, 128), 1u);
+                                    smem_desc(bh + boff, 1024, 128), 1u, kIdescF16);
                         }
                     }
                     mma_commit(bmma);
