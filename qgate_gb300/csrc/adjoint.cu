@@ -59,9 +59,9 @@ template <class R> __device__ __forceinline__ R warp_sum(R v) {
 
 template <class R, int RL, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? 256 : 512)
-k_adj_stage(typename CT<R>::type *__restrict__ psi_all, typename CT<R>::type *__restrict__ lam_all,
-            const __grid_constant__ AdjStageDesc d, const R *__restrict__ mats_all,
-            R *__restrict__ gpart) {
+k_adj_stage(const typename CT<R>::type *psi_src, typename CT<R>::type *psi_dst,
+            typename CT<R>::type *lam_all, int store_lam, const __grid_constant__ AdjStageDesc d,
+            const R *__restrict__ mats_all, R *__restrict__ gpart) {
     typedef typename CT<R>::type C;
     constexpr int NR = 1 << RL;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -69,7 +69,7 @@ k_adj_stage(typename CT<R>::type *__restrict__ psi_all, typename CT<R>::type *__
     const unsigned tid = threadIdx.x, T = blockDim.x;
     const int b = blockIdx.y;
     const idx_t tiles = (idx_t)gridDim.x;
-    C *psi = psi_all + ((idx_t)b << n);
+    const C *psi = psi_src + ((idx_t)b << n);
     C *lam = MODE == 1 ? lam_all + ((idx_t)b << n) : nullptr;
 
     C *sp = (C *)smraw;
@@ -104,7 +104,10 @@ k_adj_stage(typename CT<R>::type *__restrict__ psi_all, typename CT<R>::type *__
     for (int i = 0; i < NR; ++i) {
         unsigned slot = pt ^ Swz<R>::f((unsigned)i << t);
         idx_t g = base | dt | sdep[i];
-        cp_async_elem(&sp[slot], &psi[g]);
+        if (MODE == 0 && !psi_src)
+            sp[slot] = cmk<C>(g == 0 ? 1. : 0., 0.);  // |0...0>
+        else
+            cp_async_elem(&sp[slot], &psi[g]);
         if (MODE == 1) cp_async_elem(&sl[slot], &lam[g]);
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -188,20 +191,26 @@ k_adj_stage(typename CT<R>::type *__restrict__ psi_all, typename CT<R>::type *__
         }
     }
 
+    // psi goes nowhere when a checkpoint replaces it next, lambda when no
+    // rotation is left before it
+    const bool keep_psi = MODE == 0 || psi_dst != nullptr, keep_lam = MODE == 1 && store_lam;
     __syncthreads();
+    if (keep_psi || keep_lam) {
 #pragma unroll
-    for (int j = 0; j < NR; ++j) {
-        unsigned sl_ = reg_slot<RL>(P0, q, j);
-        sp[sl_] = a[j];
-        if (MODE == 1) sl[sl_] = l[j];
-    }
-    __syncthreads();
+        for (int j = 0; j < NR; ++j) {
+            unsigned sl_ = reg_slot<RL>(P0, q, j);
+            if (keep_psi) sp[sl_] = a[j];
+            if (keep_lam) sl[sl_] = l[j];
+        }
+        __syncthreads();
+        C *out = psi_dst + ((idx_t)b << n);
 #pragma unroll
-    for (int i = 0; i < NR; ++i) {
-        unsigned slot = pt ^ Swz<R>::f((unsigned)i << t);
-        idx_t g = base | dt | sdep[i];
-        psi[g] = sp[slot];
-        if (MODE == 1) lam[g] = sl[slot];
+        for (int i = 0; i < NR; ++i) {
+            unsigned slot = pt ^ Swz<R>::f((unsigned)i << t);
+            idx_t g = base | dt | sdep[i];
+            if (keep_psi) out[g] = sp[slot];
+            if (keep_lam) lam[g] = sl[slot];
+        }
     }
     if (MODE == 1)
         for (int i = tid; i < d.ngrads; i += T)
@@ -307,8 +316,9 @@ __global__ void k_sum_rows(const double *__restrict__ partials, int cols, double
 constexpr int kPauliBlocks = 152 * 2;
 
 template <class R, int MODE>
-void adj_dispatch(void *psi, void *lam, const AdjStageDesc &d, const void *mats, void *gpart,
-                  int batch, cudaStream_t stream) {
+void adj_dispatch(const void *psi_src, void *psi_dst, void *lam, bool store_lam,
+                  const AdjStageDesc &d, const void *mats, void *gpart, int batch,
+                  cudaStream_t stream) {
     typedef typename CT<R>::type C;
     const int NRmax = 1 << d.rl;
     size_t smem = ((size_t)sizeof(C) << d.m) * (MODE == 1 ? 2 : 1) + (size_t)d.nops * sizeof(AdjOp) +
@@ -319,7 +329,8 @@ void adj_dispatch(void *psi, void *lam, const AdjStageDesc &d, const void *mats,
     dim3 grid((unsigned)tiles, (unsigned)batch);
     auto launch = [&](auto kern) {
         QG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, threads, smem, stream>>>((C *)psi, (C *)lam, d, (const R *)mats, (R *)gpart);
+        kern<<<grid, threads, smem, stream>>>((const C *)psi_src, (C *)psi_dst, (C *)lam,
+                                              store_lam ? 1 : 0, d, (const R *)mats, (R *)gpart);
     };
     switch (d.rl) {
     case 3: launch(k_adj_stage<R, 3, MODE>); break;
@@ -339,18 +350,22 @@ void adj_dispatch(void *psi, void *lam, const AdjStageDesc &d, const void *mats,
 
 }  // namespace
 
-void launch_adj_stage(int prec, int mode, void *psi, void *lam, const AdjStageDesc &d,
-                      const void *mats, void *grad_partials, int batch, cudaStream_t stream) {
+void launch_adj_stage(int prec, int mode, const void *psi_src, void *psi_dst, void *lam,
+                      bool store_lam, const AdjStageDesc &d, const void *mats,
+                      void *grad_partials, int batch, cudaStream_t stream) {
+    auto run = [&](auto dispatch) {
+        dispatch(psi_src, psi_dst, lam, store_lam, d, mats, grad_partials, batch, stream);
+    };
     if (prec == kFP32) {
         if (mode == 0)
-            adj_dispatch<float, 0>(psi, lam, d, mats, grad_partials, batch, stream);
+            run(adj_dispatch<float, 0>);
         else
-            adj_dispatch<float, 1>(psi, lam, d, mats, grad_partials, batch, stream);
+            run(adj_dispatch<float, 1>);
     } else {
         if (mode == 0)
-            adj_dispatch<double, 0>(psi, lam, d, mats, grad_partials, batch, stream);
+            run(adj_dispatch<double, 0>);
         else
-            adj_dispatch<double, 1>(psi, lam, d, mats, grad_partials, batch, stream);
+            run(adj_dispatch<double, 1>);
     }
 }
 

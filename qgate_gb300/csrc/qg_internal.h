@@ -273,11 +273,15 @@ struct AdjStageDesc {
 
 // mode 0: apply ops to psi.  mode 1: for each op, first accumulate the
 // gradient term Im<lam|P1 G|psi> of its slot (if any), then apply the op's
-// (adjoint) matrix to both psi and lam.  mats: [batch][nmats][8] in the
-// state's precision; grad_partials: [batch][ngrads][tiles] in the state's
-// precision.  States of batch element b start at b * 2^n.
-void launch_adj_stage(int prec, int mode, void *psi, void *lam, const AdjStageDesc &d,
-                      const void *mats, void *grad_partials, int batch, cudaStream_t stream);
+// (adjoint) matrix to both psi and lam.  psi is read at psi_src (mode 0:
+// nullptr is |0...0>) and written to psi_dst, which may be the same (mode 1:
+// nullptr where it is not needed any more); lam is updated in place, or left as
+// it was without store_lam.  mats: [batch][nmats][8] in the state's precision;
+// grad_partials: [batch][ngrads][tiles] in the state's precision.  States of
+// batch element b start at b * 2^n.
+void launch_adj_stage(int prec, int mode, const void *psi_src, void *psi_dst, void *lam,
+                      bool store_lam, const AdjStageDesc &d, const void *mats,
+                      void *grad_partials, int batch, cudaStream_t stream);
 // grad[b * n_params + param[s]] += scale[s] * sum_t partials[b][s][t]  (FP64)
 void launch_adj_grad_reduce(int prec, const void *partials, int batch, int nslots, idx_t tiles,
                             const int *d_param, const double *d_scale, double *grad,
