@@ -289,6 +289,170 @@ k_marginal(double *__restrict__ out, int n_lanes, idx_t hidden_per_group,
     }
 }
 
+// ------------------------------------------------------------ one state
+
+// Bit of a tile index at lane `lane` of the warp, spread to its position.
+struct TileBits {
+    signed char pos[32];  // position of tile-index bit i
+};
+__device__ __forceinline__ idx_t spread_bits(unsigned tile, const TileBits &tb, unsigned lane) {
+    const bool on = tile >> lane & 1u;
+    const int p = tb.pos[lane];
+    const unsigned lo = on && p < 32 ? 1u << p : 0u;
+    const unsigned hi = on && p >= 32 ? 1u << (p - 32) : 0u;
+    return (idx_t)(((unsigned long long)__reduce_or_sync(0xffffffffu, hi) << 32) |
+                   __reduce_or_sync(0xffffffffu, lo));
+}
+
+// Lane permutation of one state over an aligned range of 2^k external indices:
+// out[i] = op(psi[local(start + i)]).  A tile holds ten lanes, among them the
+// lowest five of the state (loads in runs of 32 amplitudes) and the lanes of
+// the lowest five external bits (stores in runs of 32 values), and turns
+// around in shared memory.  Bound by HBM: one read, one write; a thread per
+// value with its own lane map (k_gather) reads a 32-byte sector per amplitude
+// where the low external bits are high lanes: the probability vector of 25
+// complex128 lanes in reversed order took 0.87 ms.
+constexpr int kPermLanes = 10;
+struct PermDesc {
+    idx_t src0;                    // amplitude index of the range's fixed bits
+    signed char in_pos[kPermLanes];   // ascending lanes of the tile
+    signed char out_pos[kPermLanes];  // ascending external bits of the tile
+    unsigned short in_bit[kPermLanes];  // tile-index bit (load order) of store-order bit k
+    int tiles_log2;
+    TileBits in_tile, out_tile;
+};
+__device__ __forceinline__ unsigned perm_slot(unsigned e) { return e ^ (e >> 5); }
+
+template <class R, int MATHOP> struct PermOut;
+template <class R> struct PermOut<R, 0> {
+    typedef typename CT<R>::type T;
+    static __device__ __forceinline__ T f(typename CT<R>::type c) { return c; }
+};
+template <class R> struct PermOut<R, 1> {
+    typedef R T;
+    static __device__ __forceinline__ T f(typename CT<R>::type c) { return c.x * c.x + c.y * c.y; }
+};
+template <class R> struct PermOut<R, 2> {  // FP64 of the probability in the state's precision
+    typedef double T;
+    static __device__ __forceinline__ T f(typename CT<R>::type c) { return (double)abs2r(c); }
+};
+
+template <class R, int MATHOP>
+__global__ void __launch_bounds__(256)
+k_permute(typename PermOut<R, MATHOP>::T *__restrict__ out,
+          const typename CT<R>::type *__restrict__ psi, const __grid_constant__ PermDesc d) {
+    typedef PermOut<R, MATHOP> Op;
+    __shared__ typename Op::T sm[1 << kPermLanes];
+    const unsigned tid = threadIdx.x, lane = tid & 31u;
+    // this thread's values: load order tid + 256 u, store order tid + 256 u
+    idx_t in0 = 0, out0 = 0;
+    unsigned slot0 = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (tid >> k & 1u) {
+            in0 |= 1LL << d.in_pos[k];
+            out0 |= 1LL << d.out_pos[k];
+            slot0 ^= d.in_bit[k];
+        }
+    const idx_t in8 = 1LL << d.in_pos[8], in9 = 1LL << d.in_pos[9];
+    const idx_t out8 = 1LL << d.out_pos[8], out9 = 1LL << d.out_pos[9];
+    psi += d.src0;
+    for (unsigned t = blockIdx.x; t < 1u << d.tiles_log2; t += gridDim.x) {
+        const typename CT<R>::type *p = psi + (spread_bits(t, d.in_tile, lane) | in0);
+        const typename CT<R>::type c0 = p[0], c1 = p[in8], c2 = p[in9], c3 = p[in8 + in9];
+        __syncthreads();  // the tile before is stored
+        sm[perm_slot(tid)] = Op::f(c0);
+        sm[perm_slot(tid + 256u)] = Op::f(c1);
+        sm[perm_slot(tid + 512u)] = Op::f(c2);
+        sm[perm_slot(tid + 768u)] = Op::f(c3);
+        __syncthreads();
+        typename Op::T *o = out + (spread_bits(t, d.out_tile, lane) | out0);
+        o[0] = sm[perm_slot(slot0)];
+        o[out8] = sm[perm_slot(slot0 ^ d.in_bit[8])];
+        o[out9] = sm[perm_slot(slot0 ^ d.in_bit[9])];
+        o[out8 + out9] = sm[perm_slot(slot0 ^ d.in_bit[8] ^ d.in_bit[9])];
+    }
+}
+
+// Marginal of one state with hidden lanes.  A CTA streams runs of 256
+// contiguous amplitudes (the lowest eight lanes) over the hidden ones of the
+// higher lanes, eight loads in flight per thread, one FP64 sum per thread, and
+// at the end adds the threads that differ in hidden low lanes.  CTAs: the
+// visible high lanes, times groups of hidden ones where that leaves the GPU
+// idle.  Bound by the FP64 adds (complex128: two multiply-adds per amplitude at
+// two operations per cycle and SM; complex64: one add) or HBM.  One thread per
+// output with its own lane map (k_marginal) took 0.39 ms for 15 of 25
+// complex128 lanes, whose bytes take 0.08 ms.
+struct MargDesc {
+    int nvis, nhid;               // visible / hidden lanes above the lowest eight
+    signed char vis_pos[kMaxLanes], vis_ext[kMaxLanes], hid_pos[kMaxLanes];
+    signed char low_ext[8];       // external bit of lanes 0..7 (-1: hidden)
+    int groups_log2;              // of the hidden range
+};
+template <class R> __device__ __forceinline__ void add_abs2(double &acc, typename CT<R>::type c) {
+    if constexpr (sizeof(R) == 8) {
+        acc = fma(c.x, c.x, acc);
+        acc = fma(c.y, c.y, acc);
+    } else {
+        acc += (double)abs2r(c);
+    }
+}
+template <class R>
+__global__ void __launch_bounds__(256)
+k_marginal_stream(double *__restrict__ out, idx_t n_out, const typename CT<R>::type *__restrict__ psi,
+                  const __grid_constant__ MargDesc d) {
+    __shared__ double sm[256];
+    const unsigned tid = threadIdx.x;
+    idx_t base = tid, o = 0;
+    for (int k = 0; k < d.nvis; ++k)
+        if (blockIdx.x >> k & 1u) {
+            base |= 1LL << d.vis_pos[k];
+            o |= 1LL << d.vis_ext[k];
+        }
+    // the group's hidden bits are the upper ones; the lowest three are unrolled
+    const int mine = d.nhid - d.groups_log2;
+    for (int k = 0; k < d.groups_log2; ++k)
+        if (blockIdx.y >> k & 1u) base |= 1LL << d.hid_pos[mine + k];
+    double acc = 0.;
+    if (mine < 3) {
+        for (unsigned c = 0; c < 1u << mine; ++c) {
+            idx_t off = 0;
+            for (int k = 0; k < mine; ++k)
+                if (c >> k & 1u) off |= 1LL << d.hid_pos[k];
+            add_abs2<R>(acc, psi[base + off]);
+        }
+    } else {
+        const idx_t h0 = 1LL << d.hid_pos[0], h1 = 1LL << d.hid_pos[1], h2 = 1LL << d.hid_pos[2];
+        const idx_t last = (idx_t)1 << (mine - 3);
+        idx_t off = 0;
+        for (idx_t c = 0; c < last; ++c) {  // Gray-code order: one lane flips
+            const typename CT<R>::type *p = psi + base + off;
+            typename CT<R>::type v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                v[u] = p[(u & 1 ? h0 : 0) + (u & 2 ? h1 : 0) + (u & 4 ? h2 : 0)];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) add_abs2<R>(acc, v[u]);
+            off ^= 1LL << d.hid_pos[2 + (c + 1 < last ? __ffsll(c + 1) : 1)];
+        }
+    }
+    sm[tid] = acc;
+    __syncthreads();
+    bool writes = true;
+    for (int b = 0; b < 8; ++b) {
+        if (d.low_ext[b] >= 0) {
+            if (tid >> b & 1u) o |= 1LL << d.low_ext[b];
+            continue;
+        }
+        if (tid >> b & 1u) writes = false;
+        const double other = sm[tid ^ (1u << b)];
+        __syncthreads();
+        sm[tid] += other;
+        __syncthreads();
+    }
+    if (writes) out[(idx_t)blockIdx.y * n_out + o] = sm[tid];
+}
+
 __global__ void k_sum_groups(double *__restrict__ out, const double *__restrict__ parts,
                              idx_t n_out, int n_groups) {
     const idx_t stride = (idx_t)gridDim.x * blockDim.x;
@@ -864,6 +1028,61 @@ void launch_pauli(int prec, const void *state, int n_lanes, unsigned long long x
     QG_CUDA(cudaGetLastError());
 }
 
+// The permutation descriptor of one state over external indices [start, start +
+// count): false where the form is another (several states, a range that is not
+// an aligned power of two, fewer than ten free lanes, repeated external bits, an
+// external bit of the range that no lane has).
+static bool perm_desc(const GatherDesc &g, idx_t start, idx_t count, PermDesc *d) {
+    if (g.nqs != 1 || start < 0 || count < ((idx_t)1 << kPermLanes) || (count & (count - 1)) ||
+        (start & (count - 1)))
+        return false;
+    const int k = 63 - __builtin_clzll((unsigned long long)count);
+    const int n = g.lane_begin[1] - g.lane_begin[0];
+    if (k > n || k - kPermLanes > 31) return false;
+    int lane_of[64];
+    for (int e = 0; e < 64; ++e) lane_of[e] = -1;
+    d->src0 = 0;
+    for (int l = 0; l < n; ++l) {
+        const int e = g.ext[g.lane_begin[0] + l];
+        if (lane_of[e] >= 0) return false;
+        lane_of[e] = l;
+        if (e >= k && (start >> e & 1)) d->src0 |= 1LL << l;
+    }
+    int free_lane[64], nfree = 0, ext_of[64];
+    for (int l = 0; l < 64; ++l) ext_of[l] = -1;
+    for (int e = 0; e < k; ++e) {
+        if (lane_of[e] < 0) return false;
+        ext_of[lane_of[e]] = e;
+    }
+    for (int l = 0; l < n; ++l)
+        if (ext_of[l] >= 0) free_lane[nfree++] = l;
+    unsigned long long tile = 0;
+    for (int i = 0; i < 5; ++i) tile |= 1ULL << free_lane[i] | 1ULL << lane_of[i];
+    for (int i = 0; __builtin_popcountll(tile) < kPermLanes; ++i) tile |= 1ULL << free_lane[i];
+    int ni = 0, nt = 0;
+    unsigned long long ext_tile = 0;
+    int tile_bit[64];
+    for (int i = 0; i < nfree; ++i)
+        if (tile >> free_lane[i] & 1) {
+            tile_bit[free_lane[i]] = ni;
+            d->in_pos[ni++] = (signed char)free_lane[i];
+            ext_tile |= 1ULL << ext_of[free_lane[i]];
+        }
+    for (int i = 0; i < 32; ++i) d->in_tile.pos[i] = d->out_tile.pos[i] = 0;
+    int no = 0;
+    for (int e = 0; e < k; ++e) {
+        if (ext_tile >> e & 1) {
+            d->out_pos[no] = (signed char)e;
+            d->in_bit[no++] = (unsigned short)(1u << tile_bit[lane_of[e]]);
+        } else {
+            d->out_tile.pos[nt] = (signed char)e;
+            d->in_tile.pos[nt++] = (signed char)lane_of[e];
+        }
+    }
+    d->tiles_log2 = nt;
+    return true;
+}
+
 void launch_gather(int prec, int mathop, void *out, idx_t count, idx_t start, idx_t step,
                    unsigned long long empty_mask, const GatherDesc &g, cudaStream_t stream) {
     if (count <= 0) return;
@@ -887,6 +1106,25 @@ void launch_gather(int prec, int mathop, void *out, idx_t count, idx_t start, id
                 k_gather_contig<double, 0><<<nq, 256, 0, stream>>>(out, p, count);
             else
                 k_gather_contig<double, 1><<<nq, 256, 0, stream>>>(out, p, count);
+        }
+        QG_CUDA(cudaGetLastError());
+        return;
+    }
+    PermDesc pd;
+    if (step == 1 && empty_mask == 0 && perm_desc(g, start, count, &pd)) {
+        const unsigned np = (unsigned)std::min<idx_t>((idx_t)1 << pd.tiles_log2, 152 * 8);
+        if (prec == kFP32) {
+            if (mathop == 0)
+                k_permute<float, 0><<<np, 256, 0, stream>>>((float2 *)out, (const float2 *)g.ptr[0], pd);
+            else
+                k_permute<float, 1><<<np, 256, 0, stream>>>((float *)out, (const float2 *)g.ptr[0], pd);
+        } else {
+            if (mathop == 0)
+                k_permute<double, 0><<<np, 256, 0, stream>>>((double2 *)out,
+                                                             (const double2 *)g.ptr[0], pd);
+            else
+                k_permute<double, 1><<<np, 256, 0, stream>>>((double *)out,
+                                                             (const double2 *)g.ptr[0], pd);
         }
         QG_CUDA(cudaGetLastError());
         return;
@@ -921,8 +1159,69 @@ size_t marginal_scratch_doubles(int n_lanes, int n_hidden) {
     return ((size_t)1 << gl) << n_lanes;
 }
 
+// The one-state forms: a permutation where nothing is hidden, else the streaming
+// sum.  False where the form is another (several states, external lanes that
+// repeat or leave gaps, fewer than 12 lanes).
+static bool marginal_one_state(int prec, double *out, int n_lanes, int n_hidden,
+                               const GatherDesc &g, double *d_scratch, size_t scratch_doubles,
+                               cudaStream_t stream) {
+    const int n = n_lanes + n_hidden;
+    if (g.nqs != 1 || g.lane_begin[1] - g.lane_begin[0] != n || n < 12) return false;
+    unsigned long long seen = 0;
+    for (int l = 0; l < n; ++l) {
+        const int e = g.ext[l];
+        if (e >= n || (seen >> e & 1)) return false;
+        seen |= 1ULL << e;
+    }
+    const idx_t n_out = (idx_t)1 << n_lanes;
+    PermDesc pd;
+    if (n_hidden == 0) {
+        if (!perm_desc(g, 0, n_out, &pd)) return false;
+        const unsigned np = (unsigned)std::min<idx_t>((idx_t)1 << pd.tiles_log2, 152 * 8);
+        if (prec == kFP32)
+            k_permute<float, 2><<<np, 256, 0, stream>>>(out, (const float2 *)g.ptr[0], pd);
+        else
+            k_permute<double, 2><<<np, 256, 0, stream>>>(out, (const double2 *)g.ptr[0], pd);
+        QG_CUDA(cudaGetLastError());
+        return true;
+    }
+    MargDesc d;
+    d.nvis = d.nhid = 0;
+    for (int l = 0; l < n; ++l) {
+        const int e = g.ext[l];
+        if (l < 8) {
+            d.low_ext[l] = (signed char)(e < n_lanes ? e : -1);
+        } else if (e < n_lanes) {
+            d.vis_pos[d.nvis] = (signed char)l;
+            d.vis_ext[d.nvis++] = (signed char)e;
+        } else {
+            d.hid_pos[d.nhid++] = (signed char)l;
+        }
+    }
+    if (d.nvis > 24) return false;
+    // enough CTAs to fill the GPU evenly (8192, seven waves), each with at least
+    // eight runs, and no more partial sums than the scratch holds
+    int gl = 0;
+    while (d.nvis + gl < 13 && d.nhid - gl > 3 && (((size_t)2 << gl) << n_lanes) <= scratch_doubles)
+        ++gl;
+    d.groups_log2 = gl;
+    double *dst = gl == 0 ? out : d_scratch;
+    const dim3 grid(1u << d.nvis, 1u << gl);
+    if (prec == kFP32)
+        k_marginal_stream<float><<<grid, 256, 0, stream>>>(dst, n_out, (const float2 *)g.ptr[0], d);
+    else
+        k_marginal_stream<double><<<grid, 256, 0, stream>>>(dst, n_out, (const double2 *)g.ptr[0], d);
+    if (gl != 0)
+        k_sum_groups<<<sm_grid(n_out, 256, 152 * 16), 256, 0, stream>>>(out, d_scratch, n_out,
+                                                                       1 << gl);
+    QG_CUDA(cudaGetLastError());
+    return true;
+}
+
 void launch_marginal(int prec, double *out, int n_lanes, int n_hidden, const GatherDesc &g,
                      double *d_scratch, size_t scratch_doubles, cudaStream_t stream) {
+    if (marginal_one_state(prec, out, n_lanes, n_hidden, g, d_scratch, scratch_doubles, stream))
+        return;
     int gl = marginal_groups(n_lanes, n_hidden);
     idx_t n_out = (idx_t)1 << n_lanes;
     int identity = 0;
