@@ -20,6 +20,8 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <exception>
+#include <mutex>
 #include <vector>
 
 namespace qg {
@@ -322,97 +324,190 @@ void build_launches(const std::vector<Op> &ops, const std::vector<int> &order, i
 // planned like the gate queue's (plan_stage_lanes over 12-lane tiles); the
 // lanes, blocks and layouts depend only on the gates' lanes, so they are the
 // same for every parameter vector, and only the block unitaries differ: one
-// k_tstage launch per stage and vector, each with that vector's operands.
+// k_tstage launch per stage, over all vectors with each vector's operands.
 struct TcForward {
     struct Step {
         TcStageDesc desc;     // bmats filled at launch
-        size_t ops_off;       // byte offset of batch element 0's operands
+        TcLaunchOrder order;
+        TileLanes tl;
+        std::vector<std::pair<unsigned, std::vector<int>>> ops;  // lanes, gates (op indices)
         size_t ops_stride;    // operand bytes per batch element
-        int ckpt_after;       // save psi to this checkpoint after the step (-1: none)
+        int ckpt_after;       // write this checkpoint in place of psi (-1: none)
     };
     std::vector<Step> steps;
-    std::vector<unsigned char> ops;  // [step][batch][nb][Bh | Bl]
 };
 
-void plan_tc_forward(const std::vector<Op> &ops, const std::vector<int> &bounds, int n, int batch,
-                     int n_params, const double *params, TcForward &out) {
+// Loop bodies on the host threads, which an exception must not leave.
+class FirstError {
+public:
+    template <class F>
+    void run(F &&body) {
+        try {
+            body();
+        } catch (...) {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (!e_) e_ = std::current_exception();
+        }
+    }
+    void rethrow() {
+        if (e_) std::rethrow_exception(e_);
+    }
+
+private:
+    std::mutex mu_;
+    std::exception_ptr e_;
+};
+
+struct CopyEvent {
+    cudaEvent_t e = nullptr;
+    CopyEvent() { QG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
+    ~CopyEvent() { cudaEventDestroy(e); }
+    CopyEvent(const CopyEvent &) = delete;
+};
+
+PendingGate gate_of(const Op &o, const double *params) {
+    PendingGate g;
+    g.target = o.target;
+    g.controls = o.controls;
+    if (o.kind == 1)
+        rotation(o.axis, o.coef * params[o.param], g.m.v);
+    else
+        memcpy(g.m.v, o.mat, sizeof(g.m.v));
+    g.diag = is_diag(g.m);
+    return g;
+}
+
+void plan_tc_forward(const std::vector<Op> &ops, const std::vector<int> &bounds, int n,
+                     const double *params, TcForward &out) {
     const int M = 12;
     const unsigned long long base = (1ULL << 4) - 1;
-    auto gate_of = [&](const Op &o, int b) {
-        PendingGate g;
-        g.target = o.target;
-        g.controls = o.controls;
-        if (o.kind == 1)
-            rotation(o.axis, o.coef * params[(size_t)b * n_params + o.param], g.m.v);
-        else
-            memcpy(g.m.v, o.mat, sizeof(g.m.v));
-        g.diag = is_diag(g.m);
-        return g;
-    };
     const int nseg = (int)bounds.size() - 1;
-    for (int sgi = 0; sgi < nseg; ++sgi) {
+    std::vector<std::vector<TcForward::Step>> segs(nseg);
+    auto plan_segment = [&](int sgi) {
         // planning on batch element 0's gates (only their lanes matter)
         std::vector<PendingGate> g0;
-        for (int j = bounds[sgi]; j < bounds[sgi + 1]; ++j) g0.push_back(gate_of(ops[j], 0));
+        for (int j = bounds[sgi]; j < bounds[sgi + 1]; ++j) g0.push_back(gate_of(ops[j], params));
         std::vector<const PendingGate *> remaining;
         for (auto &g : g0) remaining.push_back(&g);
+        std::vector<unsigned char> scratch;
         while (!remaining.empty()) {
             unsigned long long S = plan_stage_lanes(remaining, base, M);
             std::vector<const PendingGate *> chosen, deferred;
             stage_take(remaining, S, remaining.size(), &chosen, &deferred);
             for (int q = 0; q < n && __builtin_popcountll(S) < M; ++q) S |= 1ULL << q;
             const TileLanes tl = tile_lanes_of(S, n);
-            const TcBlocks blocks0 = tc_blocks(chosen, tl);
-            // the blocks as indices into the segment's gates
-            std::vector<std::pair<unsigned, std::vector<int>>> bidx;
-            for (auto &bl : blocks0) {
-                std::vector<int> ix;
-                for (auto *g : bl.second) ix.push_back((int)(g - g0.data()));
-                bidx.emplace_back(bl.first, ix);
-            }
             // dense ops only: whether a rotation is diagonal depends on its
             // angle, which differs between parameter vectors
-            const TcOps ops0 = tc_ops(blocks0, false);
-            for (size_t b0 = 0; b0 < bidx.size();) {
+            const TcOps ops0 = tc_ops(tc_blocks(chosen, tl), false);
+            for (size_t b0 = 0; b0 < ops0.size();) {
                 const int nb = tc_ops_per_launch(ops0, b0);
                 TcForward::Step st;
-                st.ops_off = out.ops.size();
+                st.tl = tl;
                 st.ops_stride = (size_t)nb * tc_op_bytes(ops0[b0]);
                 st.ckpt_after = -1;
-                out.ops.resize(out.ops.size() + (size_t)batch * st.ops_stride);
-                std::vector<TcStageDesc> descs(batch);
-#pragma omp parallel for schedule(dynamic, 1)
-                for (int b = 0; b < batch; ++b) {
-                    std::vector<PendingGate> gb;
-                    gb.reserve(g0.size());
-                    for (int j = bounds[sgi]; j < bounds[sgi + 1]; ++j) gb.push_back(gate_of(ops[j], b));
-                    TcBlocks blocks;
-                    for (auto &bi : bidx) {
-                        std::vector<const PendingGate *> ptrs;
-                        for (int ix : bi.second) ptrs.push_back(&gb[ix]);
-                        blocks.emplace_back(bi.first, ptrs);
-                    }
-                    tc_plan_launch(tl, n, tc_ops(blocks, false), b0, nb, descs[b],
-                                   out.ops.data() + st.ops_off + (size_t)b * st.ops_stride);
+                for (int k = 0; k < nb; ++k) {
+                    std::vector<int> ix;
+                    for (auto *g : ops0[b0 + k].gates) ix.push_back(bounds[sgi] + (int)(g - g0.data()));
+                    st.ops.emplace_back(ops0[b0 + k].lanes, std::move(ix));
                 }
-                st.desc = descs[0];
-                out.steps.push_back(st);
+                scratch.resize(st.ops_stride);
+                tc_plan_launch(tl, n, ops0, b0, nb, st.desc, scratch.data(), kFP32, &st.order);
+                segs[sgi].push_back(std::move(st));
                 b0 += nb;
             }
             remaining.swap(deferred);
         }
-        if (sgi + 1 < nseg && !out.steps.empty()) out.steps.back().ckpt_after = sgi;
-    }
+        if (sgi + 1 < nseg && !segs[sgi].empty()) segs[sgi].back().ckpt_after = sgi;
+    };
+    FirstError err;
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int sgi = 0; sgi < nseg; ++sgi) err.run([&] { plan_segment(sgi); });
+    err.rethrow();
+    for (auto &s : segs)
+        for (auto &st : s) out.steps.push_back(std::move(st));
 }
 
-// A tensor forward stage is one launch per parameter vector, of 2^(n-14) CTAs,
-// and its operands are formed on the host for each; the CUDA-core stage is one
-// launch for all vectors.  Measured (forward sweep, 6 layers, batch 16, CUDA cores
-// against tensor): 20 qubits 4.6 against 10.1 ms without checkpoints and 10.2
-// against 37.6 ms with one every 3 gates, 14 qubits 1.5 against 24.4 ms; with 24
-// qubits, which fill the GPU by themselves, 12 layers and a checkpoint every 3
-// layers the tensor forward makes the whole call 10 % faster.
-bool tc_forward_pays(int n, int gates_per_segment) { return n >= 23 && gates_per_segment >= 64; }
+// One vector's operands of a step.
+void tc_forward_operands(const TcForward::Step &st, const std::vector<PendingGate> &gates,
+                         unsigned char *buf) {
+    TcOps o;
+    for (auto &bl : st.ops) {
+        TcOp op;
+        op.phase = false;
+        op.lanes = bl.first;
+        for (int ix : bl.second) op.gates.push_back(&gates[ix]);
+        o.push_back(std::move(op));
+    }
+    tc_launch_operands(st.tl, o, 0, (int)o.size(), st.desc, st.order, buf);
+}
+
+// Runs the forward sweep from |0...0>: the operands are formed on the host
+// threads into one half of a pinned buffer while the device runs on the other
+// half's.  A stage's launch covers every vector (2^(n-14) CTAs each would leave
+// most SMs idle up to 20 qubits), and a checkpoint is written by the stage
+// before it and read by the stage after it, without a copy.  Measured, forward
+// sweep, 20 qubits, 6 layers, batch 16: 37.6 -> 10.1 ms with a checkpoint every 3 gates (whole gradient 62.5 ->
+// 22.6 ms), 10.1 -> 8.7 without; 14 qubits, 23.5 -> 3.7 ms.
+void run_tc_forward(const std::vector<Op> &ops, const std::vector<int> &bounds, int n, int batch,
+                    int n_params, const double *params, char *psi, char *ck, cudaStream_t st,
+                    std::vector<void *> &owned) {
+    const size_t vec_bytes = (size_t)8 << n;
+    TcForward f;
+    plan_tc_forward(ops, bounds, n, params, f);
+    for (int b = 0; b < batch; ++b)
+        launch_init_basis(kFP32, psi + vec_bytes * b, (idx_t)1 << n, st);
+    if (f.steps.empty()) return;
+    FirstError err;
+    std::vector<std::vector<PendingGate>> gates(batch);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int b = 0; b < batch; ++b)
+        err.run([&] {
+            for (auto &o : ops) gates[b].push_back(gate_of(o, params + (size_t)b * n_params));
+        });
+    err.rethrow();
+    size_t half = (size_t)2 << 20;
+    for (auto &s : f.steps) half = std::max(half, s.ops_stride * batch);
+    unsigned char *host = (unsigned char *)engine_pinned(2 * half);
+    unsigned char *devb = (unsigned char *)engine_alloc(2 * half);
+    owned.push_back(devb);
+    CopyEvent done[2];
+    char *cur = psi;
+    int which = 0;
+    for (size_t s0 = 0; s0 < f.steps.size(); which ^= 1) {
+        size_t s1 = s0, bytes = 0;
+        std::vector<size_t> at;
+        for (; s1 < f.steps.size() && bytes + f.steps[s1].ops_stride * batch <= half; ++s1) {
+            at.push_back(bytes);
+            bytes += f.steps[s1].ops_stride * batch;
+        }
+        unsigned char *hb = host + which * half, *db = devb + which * half;
+        QG_CUDA(cudaEventSynchronize(done[which].e));  // the copy two rounds ago
+        const int jobs = (int)(s1 - s0) * batch;
+#pragma omp parallel for schedule(dynamic, 4)
+        for (int j = 0; j < jobs; ++j) {
+            err.run([&] {
+                const TcForward::Step &s = f.steps[s0 + j / batch];
+                tc_forward_operands(s, gates[j % batch],
+                                    hb + at[j / batch] + (size_t)(j % batch) * s.ops_stride);
+            });
+        }
+        err.rethrow();
+        QG_CUDA(cudaMemcpyAsync(db, hb, bytes, cudaMemcpyHostToDevice, st));
+        QG_CUDA(cudaEventRecord(done[which].e, st));
+        for (size_t s = s0; s < s1; ++s) {
+            TcStageDesc d = f.steps[s].desc;
+            char *dst = ck && f.steps[s].ckpt_after >= 0
+                            ? ck + vec_bytes * batch * f.steps[s].ckpt_after : psi;
+            for (int b = 0; b < batch; b += 32768) {
+                d.bmats = db + at[s - s0] + (size_t)b * f.steps[s].ops_stride;
+                launch_tstage(dst + vec_bytes * b, d, st, false, cur + vec_bytes * b,
+                              std::min(batch - b, 32768), f.steps[s].ops_stride);
+            }
+            cur = dst;
+        }
+        s0 = s1;
+    }
+}
 
 }  // namespace
 
@@ -448,13 +543,9 @@ static void adjoint_run(int prec, int n, std::vector<Op> &ops, const double *par
     std::vector<R> mats;
     std::vector<int> slot_param;
     std::vector<double> slot_scale;
-    // complex64 forward sweeps run on the tensor cores where that is faster
-    const bool tc_fwd = sizeof(R) == 4 && n >= 13 && tensor_stages_enabled() &&
-                        tc_forward_pays(n, N / nseg);
-    TcForward tcf;
-    if (tc_fwd) {
-        plan_tc_forward(ops, bounds, n, batch, n_params, params, tcf);
-    } else {
+    // complex64 forward sweeps run on the tensor cores
+    const bool tc_fwd = sizeof(R) == 4 && n >= 13 && tensor_stages_enabled();
+    if (!tc_fwd) {
         for (int s = 0; s < nseg; ++s) {
             std::vector<int> order;
             for (int j = bounds[s]; j < bounds[s + 1]; ++j) order.push_back(j);
@@ -466,17 +557,6 @@ static void adjoint_run(int prec, int n, std::vector<Op> &ops, const double *par
         }
     }
     const size_t n_fwd = launches.size();
-    if (G_out) {
-        for (int s = nseg - 1; s >= 0; --s) {
-            std::vector<int> order;
-            for (int j = bounds[s + 1] - 1; j >= bounds[s]; --j) order.push_back(j);
-            size_t first = launches.size();
-            build_launches<R>(ops, order, n, M_bwd, rl_b, budget, 1, batch, n_params, params,
-                              launches, mats, slot_param, slot_scale);
-            if (s + 1 < nseg && launches.size() > first) launches[first].ckpt_before = s;
-        }
-    }
-
     const int nck = nseg - 1;
     std::vector<void *> owned;
     auto alloc = [&](size_t bytes) {
@@ -488,6 +568,19 @@ static void adjoint_run(int prec, int n, std::vector<Op> &ops, const double *par
         void *psi = alloc(state_bytes * batch);
         void *lam = alloc(state_bytes * batch);
         void *ck = nck > 0 && G_out ? alloc(state_bytes * batch * nck) : nullptr;
+        if (tc_fwd)
+            run_tc_forward(ops, bounds, n, batch, n_params, params, (char *)psi, (char *)ck, st,
+                           owned);
+        if (G_out) {  // planned while the device runs the forward sweep
+            for (int s = nseg - 1; s >= 0; --s) {
+                std::vector<int> order;
+                for (int j = bounds[s + 1] - 1; j >= bounds[s]; --j) order.push_back(j);
+                size_t first = launches.size();
+                build_launches<R>(ops, order, n, M_bwd, rl_b, budget, 1, batch, n_params, params,
+                                  launches, mats, slot_param, slot_scale);
+                if (s + 1 < nseg && launches.size() > first) launches[first].ckpt_before = s;
+            }
+        }
         void *dmats = alloc(std::max<size_t>(mats.size() * sizeof(R), 16));
         QG_CUDA(cudaMemcpyAsync(dmats, mats.data(), mats.size() * sizeof(R), cudaMemcpyHostToDevice,
                                 st));
@@ -514,24 +607,6 @@ static void adjoint_run(int prec, int n, std::vector<Op> &ops, const double *par
         double *dE = (double *)alloc(sizeof(double) * batch);
 
         auto checkpoint = [&](int s) { return (void *)((char *)ck + state_bytes * batch * s); };
-        if (tc_fwd) {
-            // |0...0> for every batch element
-            for (int b = 0; b < batch; ++b)
-                launch_init_basis(prec, (char *)psi + state_bytes * b, (idx_t)1 << n, st);
-            unsigned char *dops = (unsigned char *)alloc(std::max<size_t>(tcf.ops.size(), 16));
-            QG_CUDA(cudaMemcpyAsync(dops, tcf.ops.data(), tcf.ops.size(),
-                                    cudaMemcpyHostToDevice, st));
-            for (auto &step : tcf.steps) {
-                TcStageDesc d = step.desc;
-                for (int b = 0; b < batch; ++b) {
-                    d.bmats = dops + step.ops_off + (size_t)b * step.ops_stride;
-                    launch_tstage((char *)psi + state_bytes * b, d, st, false);
-                }
-                if (step.ckpt_after >= 0 && ck)
-                    QG_CUDA(cudaMemcpyAsync(checkpoint(step.ckpt_after), psi, state_bytes * batch,
-                                            cudaMemcpyDeviceToDevice, st));
-            }
-        }
 
         // A checkpoint is the output of the stage before it and the input of the
         // stages after it: the forward sweep writes it in place of psi and reads
@@ -596,6 +671,7 @@ extern "C" int qg_adjoint_expectation(int prec, int n_qubits, const qg_circuit_o
                                       int checkpoint_every, double *expectations,
                                       double *gradients) {
     try {
+        std::lock_guard<std::recursive_mutex> lk(engine_mutex());
         if (prec != kFP32 && prec != kFP64) fail(QG_ERR_VALUE, "unexpected dtype.");
         if (n_qubits < 1 || n_qubits > 34) fail(QG_ERR_VALUE, "n_qubits out of range.");
         if (batch < 1) fail(QG_ERR_VALUE, "batch must be >= 1.");

@@ -322,6 +322,18 @@ cudaStream_t engine_stream() { return dev().stream; }
 void *engine_alloc(size_t bytes) { return dev().arena.alloc(bytes); }
 bool tensor_stages_enabled() { return dev().tensor_blocks; }
 void engine_free(void *p) { g_dev.arena.release(p); }
+std::recursive_mutex &engine_mutex() { return g_dev.mu; }
+void *engine_pinned(size_t bytes) {
+    Device &d = dev();
+    if (d.h_batch_bytes < bytes) {
+        if (d.h_batch) QG_CUDA(cudaFreeHost(d.h_batch));
+        d.h_batch = nullptr;
+        d.h_batch_bytes = 0;
+        QG_CUDA(cudaMallocHost(&d.h_batch, bytes));
+        d.h_batch_bytes = bytes;
+    }
+    return d.h_batch;
+}
 
 template <class T> static T *lookup(std::unordered_set<T *> &set, qg_handle h, const char *what) {
     T *p = reinterpret_cast<T *>(h);
@@ -2431,13 +2443,7 @@ int qg_batch_sum_z(int prec, int n_circuits, const int *n_qubits, const int64_t 
     const size_t ops_bytes = (size_t)ops_at[n_circuits] * sizeof(RegOp<float>);
     const size_t sets_bytes = (size_t)sets_at[n_circuits] * sizeof(SetSlots);
     const size_t stage_bytes = ((ops_bytes + 255) & ~(size_t)255) + sets_bytes;
-    if (d.h_batch_bytes < stage_bytes) {
-        if (d.h_batch) QG_CUDA(cudaFreeHost(d.h_batch));
-        d.h_batch = nullptr;
-        d.h_batch_bytes = 0;
-        QG_CUDA(cudaMallocHost(&d.h_batch, stage_bytes));
-        d.h_batch_bytes = stage_bytes;
-    }
+    engine_pinned(stage_bytes);
     RegOp<float> *ops_all = (RegOp<float> *)d.h_batch;
     SetSlots *sets_all = (SetSlots *)(d.h_batch + ((ops_bytes + 255) & ~(size_t)255));
 #pragma omp parallel for schedule(dynamic, 64)

@@ -10,6 +10,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <mutex>
 #include <stdint.h>
 #include <string>
 #include <vector>
@@ -197,7 +198,10 @@ struct TcStageDesc {
 };
 // two_per_row: the 12-lane variant with two threads per tile row (twice the
 // warps per SM, half the registers per thread).
-void launch_tstage(void *state, const TcStageDesc &d, cudaStream_t stream, bool two_per_row);
+// src: where the tiles are read (nullptr: in place).  batch: that many states, 2^n
+// amplitudes apart, in one launch, state b's operands at bmats + b * ops_stride.
+void launch_tstage(void *state, const TcStageDesc &d, cudaStream_t stream, bool two_per_row,
+                   const void *src = nullptr, int batch = 1, size_t ops_stride = 0);
 // The complex128 form (dstage.cu): 12-lane tiles, dense and phase ops; bmats
 // holds phase tables (tc_phase_table) and each block's digit slices: kDigitOpBytes as 8 chunks (half h, K-step ks at
 // 4 h + ks) of 160 rows x 16 FP16 values, row 32 (j - 1) + c of a chunk being
@@ -369,6 +373,10 @@ int batch_persistent_ctas();
 cudaStream_t engine_stream();
 void *engine_alloc(size_t bytes);
 void engine_free(void *p);
+// Pinned host memory of at least `bytes`, kept for the next caller; its contents
+// last until the caller's call returns.
+void *engine_pinned(size_t bytes);
+std::recursive_mutex &engine_mutex();  // held by every call that uses the engine
 
 // Descriptor of a lane-permuted gather over a product of states.
 struct GatherDesc {

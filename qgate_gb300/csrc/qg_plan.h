@@ -94,7 +94,20 @@ int tc_ops_per_launch(const TcOps &ops, size_t b0, int prec = kFP32);
 // descriptor (all but the operand pointer) and the ops' operands in `buf`
 // (dense ops first, then the phase tables; desc.ops_bytes in all).
 void tc_plan_launch(const TileLanes &tl, int n, const TcOps &ops, size_t b0, int nb,
-                    TcStageDesc &desc, unsigned char *buf, int prec = kFP32);
+                    TcStageDesc &desc, unsigned char *buf, int prec = kFP32,
+                    struct TcLaunchOrder *order = nullptr);
+
+// What the operands of a launch's dense ops depend on besides the gates'
+// matrices: which of the ops [b0, b0 + nb) runs at each place, and its block's
+// lanes in the order of the amplitude bits.  Another launch with the same lanes
+// and other matrices takes its operands from tc_launch_operands (complex64,
+// dense ops only).
+struct TcLaunchOrder {
+    int op[kMaxTcBlocks];
+    signed char amps[kMaxTcBlocks][5];
+};
+void tc_launch_operands(const TileLanes &tl, const TcOps &ops, size_t b0, int nb,
+                        const TcStageDesc &desc, const TcLaunchOrder &order, unsigned char *buf);
 
 // Whether complex64 stages run on the tensor cores (the gate queue's setting).
 bool tensor_stages_enabled();

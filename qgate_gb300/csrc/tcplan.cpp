@@ -725,7 +725,8 @@ static void tc_phase_table(const TcOp &op, const TileLanes &tl, const std::vecto
 // `tl` -> the descriptor (all but the operand pointer) and the ops' operands
 // in `buf`.
 static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops, size_t b0,
-                                   int nb, TcStageDesc &desc, unsigned char *buf, int prec);
+                                   int nb, TcStageDesc &desc, unsigned char *buf, int prec,
+                                   TcLaunchOrder *order);
 
 // Header and records of a cross op in the layout `lay` it runs in: one record
 // per gate (its two phases as angles), by the tile position of its one lane
@@ -767,8 +768,10 @@ static void tc_cross_records(const TcOp &op, const TileLanes &tl, const TcLayout
 }
 
 void tc_plan_launch(const TileLanes &tl, int n, const TcOps &ops, size_t b0, int nb,
-                    TcStageDesc &desc, unsigned char *buf, int prec) {
+                    TcStageDesc &desc, unsigned char *buf, int prec, TcLaunchOrder *order) {
     const unsigned kDirectLow = tc_direct_low(prec);
+    int at[kMaxTcBlocks];
+    for (int b = 0; b < nb; ++b) at[b] = b;
     // The launch's ops in an order that ends with a dense op leaving tile
     // positions 0..3 to the rows (its rows then go straight to the state):
     // a dense op moves to the end when it shares no lane with any op after
@@ -786,15 +789,19 @@ void tc_plan_launch(const TileLanes &tl, int n, const TcOps &ops, size_t b0, int
                 TcOp mv = slice[x];
                 slice.erase(slice.begin() + x);
                 slice.push_back(mv);
+                std::rotate(at + x, at + x + 1, at + nb);
                 break;
             }
         }
     }
-    tc_plan_launch_ordered(tl, n, slice, 0, nb, desc, buf, prec);
+    if (order)
+        for (int b = 0; b < nb; ++b) order->op[b] = at[b];
+    tc_plan_launch_ordered(tl, n, slice, 0, nb, desc, buf, prec, order);
 }
 
 static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops, size_t b0,
-                                   int nb, TcStageDesc &desc, unsigned char *buf, int prec) {
+                                   int nb, TcStageDesc &desc, unsigned char *buf, int prec,
+                                   TcLaunchOrder *order) {
     const unsigned kDirectLow = tc_direct_low(prec);
     const int m = (int)tl.lanes.size();
     const int t = m - 5;
@@ -954,6 +961,8 @@ static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops,
         }
         desc.op_kind[b] = 0;
         desc.sets[b] = tc_slots(cur, t, [&](unsigned ti) { return tc_operand_slot(lay, ti); });
+        if (order)
+            for (int k = 0; k < 5; ++k) order->amps[b][k] = (signed char)lay.amps[k];
         tc_block_matrix(op.gates, tl, lay, U);
         unsigned short *o = (unsigned short *)(buf + desc.op_off[b]);
         if (prec == kFP64) {
@@ -970,5 +979,18 @@ static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops,
     for (int k = 0; k < 5; ++k) desc.out_e[k] = 1LL << tl.lanes[cur.amps[k]];
 }
 
+
+void tc_launch_operands(const TileLanes &tl, const TcOps &ops, size_t b0, int nb,
+                        const TcStageDesc &desc, const TcLaunchOrder &order, unsigned char *buf) {
+    std::complex<double> U[1024];
+    for (int b = 0; b < nb; ++b) {
+        TcLayout lay;
+        for (int k = 0; k < 5; ++k) lay.amps[k] = order.amps[b][k];
+        tc_block_matrix(ops[b0 + order.op[b]].gates, tl, lay, U);
+        tc_compensate(U);
+        unsigned short *o = (unsigned short *)(buf + desc.op_off[b]);
+        tc_operand(U, o, o + 64 * 64);
+    }
+}
 
 }  // namespace qg

@@ -127,7 +127,8 @@ constexpr float kScale = 4096.f, kUnscale = 1.f / 4096.f;
 // the kernel keeps the registers of the dense path alone).
 template <int RT, int G, int H, bool PH>
 __global__ void __launch_bounds__(128 * RT * G * H, 1)
-k_tstage(float2 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles) {
+k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, int tiles,
+         long long state_stride, unsigned ops_stride) {
     constexpr int m = RT == 1 ? 12 : 13;
     constexpr int t = m - 5;
     constexpr int NA = 32 / H;                          // amplitudes per thread
@@ -191,7 +192,8 @@ k_tstage(float2 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tile
     const unsigned tmem = tmem_sh + g * kColsGroup + 64u * (wg >> 2) + 32u * hh +
                           ((32u * (wg & 3u)) << 16);
     const unsigned dcol0 = tmem_sh + g * kColsGroup;       // the group's accumulator
-    if (tid == 0) bulk_load(smem_u32(Bs), d.bmats, d.ops_bytes, bb);
+    if (tid == 0)
+        bulk_load(smem_u32(Bs), d.bmats + (size_t)blockIdx.y * ops_stride, d.ops_bytes, bb);
 
     // Load layout: row bit b at global lane row_lane[b], amplitude bit k at
     // the lane of e[k] (chosen per stage on the host; lanes 0..3 of the tile
@@ -217,7 +219,8 @@ k_tstage(float2 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tile
     // flight during the copy-out; the scale is applied after.
     unsigned v[2 * NA];  // floats (bits): this thread's part of row r
     auto load_raw = [&](int tl) {
-        const float2 *gp0 = s + (insert_zeros((idx_t)tl, d.ins_pos, d.nins) | row_offset());
+        const float2 *gp0 = src + blockIdx.y * state_stride +
+                            (insert_zeros((idx_t)tl, d.ins_pos, d.nins) | row_offset());
         gray_walk<NB>(gp0, e, [&](int j, const float2 *p) {
             const float2 x = *p;
             v[2 * j] = __float_as_uint(x.x);
@@ -417,7 +420,8 @@ k_tstage(float2 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tile
             for (int b = 0; b < t; ++b)
                 if (r & (1u << b)) o |= 1LL << d.out_row_lane[b];
             if (H == 2 && hh) o += d.out_e[4];
-            float2 *gp = s + (insert_zeros((idx_t)tl, d.ins_pos, d.nins) | o);
+            float2 *gp = dst + blockIdx.y * state_stride +
+                         (insert_zeros((idx_t)tl, d.ins_pos, d.nins) | o);
             gray_walk<NB>(gp, d.out_e, [&](int j, float2 *p) {
                 *p = make_float2(__uint_as_float(v[2 * j]) * kUnscale,
                                  __uint_as_float(v[2 * j + 1]) * kUnscale);
@@ -448,7 +452,8 @@ k_tstage(float2 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tile
             const SetSlots &nat = sset[nb + 1];
             unsigned slot = (unsigned)nat.lo[r & 31u] ^ (unsigned)nat.hi[r >> 5];
             if (H == 2 && hh) slot ^= nat.q[4];
-            float2 *gp = s + (insert_zeros((idx_t)tl, d.ins_pos, d.nins) | row_offset());
+            float2 *gp = dst + blockIdx.y * state_stride +
+                         (insert_zeros((idx_t)tl, d.ins_pos, d.nins) | row_offset());
             gray_walk<NB>(gp, e, [&](int j, float2 *p) {
                 const int i = gray_index(j);
                 if (i > 0) slot ^= nat.q[gray_bit(i)];
@@ -481,7 +486,10 @@ static size_t tstage_smem(int m, int groups, size_t ops_bytes, int nops) {
 // threads per row), 2 of 256 threads for 13-lane tiles.
 static int tstage_groups(int m) { return m == 12 ? 4 : 2; }
 
-void launch_tstage(void *state, const TcStageDesc &d, cudaStream_t stream, bool two_per_row) {
+void launch_tstage(void *state, const TcStageDesc &d, cudaStream_t stream, bool two_per_row,
+                   const void *src, int batch, size_t ops_stride) {
+    if (batch < 1 || batch > 65535 || (ops_stride & 15u) != 0 || ops_stride >> 32)
+        fail(2, "tensor stage: bad batch %d", batch);
     if (d.m != 12 && d.m != 13) fail(2, "tensor stage: tile lanes must be 12 or 13 (got %d)", d.m);
     if (d.nblocks < 1 || d.nblocks > kMaxTcBlocks) fail(2, "tensor stage: bad op count %d", d.nblocks);
     if (((uintptr_t)d.bmats & 15u) != 0 || (d.ops_bytes & 15u) != 0)
@@ -519,8 +527,22 @@ void launch_tstage(void *state, const TcStageDesc &d, cudaStream_t stream, bool 
     auto launch = [&](auto kern, int groups, int threads) {
         const size_t smem = tstage_smem(d.m, groups, d.ops_bytes, d.nblocks);
         QG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        const int ctas = std::min((tiles + groups - 1) / groups, sms);
-        kern<<<(unsigned)ctas, threads, smem, stream>>>((float2 *)state, d, tiles);
+        // A batch: the CTAs per state that end soonest (one CTA per SM at a time,
+        // each taking about a tile's time to start).
+        const int most = std::min((tiles + groups - 1) / groups, sms);
+        int ctas = most;
+        long long best = -1;
+        for (int x = 1; batch > 1 && x <= most; ++x) {
+            const long long waves = ((long long)x * batch + sms - 1) / sms;
+            const long long cost = waves * ((tiles + groups * x - 1) / (groups * x) + 1);
+            if (best < 0 || cost < best) {
+                best = cost;
+                ctas = x;
+            }
+        }
+        kern<<<dim3((unsigned)ctas, (unsigned)batch), threads, smem, stream>>>(
+            (const float2 *)(src ? src : state), (float2 *)state, d, tiles, 1LL << d.n,
+            (unsigned)ops_stride);
     };
     bool phases = false;  // phase or cross ops
     for (int b = 0; b < d.nblocks; ++b) phases = phases || d.op_kind[b] != 0;

@@ -1,6 +1,5 @@
-"""The adjoint engine's forward sweep on either side of its rule (tensor stages
-from 23 qubits on and 64 gates per checkpoint segment, CUDA-core stages below)
-and its checkpoints as the stages' own inputs and outputs: gradients against the
+"""The adjoint engine's tensor forward sweep, one launch per stage over all
+parameter vectors, and its checkpoints as the stages' own inputs and outputs: gradients against the
 run without tensor stages or without checkpoints (complex64 1e-5, complex128
 1e-10: the bars of test_gpu_adjoint.py)."""
 import numpy as np
@@ -17,17 +16,33 @@ def _run(n, layers, batch, dtype, every, gradient=True):
                                             gradient)
 
 
-@pytest.mark.parametrize('n,layers', [(22, 2), (23, 1), (23, 2)])
-def test_forward_rule_against_cuda_core_stages(rt, n, layers):
+# batch sizes around the SM count and sizes with fewer tiles than thread groups
+@pytest.mark.parametrize('n,layers,batch', [(13, 2, 1), (13, 2, 200), (14, 2, 152), (16, 2, 37),
+                                            (17, 1, 153), (20, 2, 5), (22, 2, 2), (23, 1, 2)])
+def test_batched_forward_against_cuda_core_stages(rt, n, layers, batch):
     from qgate_gb300 import _native as nat
-    e, g = _run(n, layers, 2, np.float32, 0)
+    e, g = _run(n, layers, batch, np.float32, 5)
     nat.set_tensor_blocks(False)
     try:
-        e0, g0 = _run(n, layers, 2, np.float32, 0)
+        e0, g0 = _run(n, layers, batch, np.float32, 5)
     finally:
         nat.set_tensor_blocks(True)
     assert np.max(np.abs(e - e0)) < 1e-5 * n
     assert np.max(np.abs(g - g0)) < 1e-5
+
+
+@pytest.mark.parametrize('n', [13, 18])
+def test_batch_is_its_vectors(rt, n):
+    """A vector's energy in a batch is the one it has alone (the forward sweep adds
+    nothing across vectors and in no other order: equal to the last bit)."""
+    from qgate_gb300 import adjoint
+    c = adjoint.hardware_efficient_ansatz(n, 2)
+    p = np.random.default_rng(n).uniform(-3, 3, (7, c.n_params))
+    h = adjoint.PauliSum.ising_chain(n)
+    e, _ = adjoint.expectation_and_gradient(c, p, h, np.float32, 3, False)
+    for b in range(7):
+        e1, _ = adjoint.expectation_and_gradient(c, p[b:b + 1], h, np.float32, 3, False)
+        assert e[b] == e1[0]
 
 
 @pytest.mark.parametrize('dtype,bar', [(np.float32, 1e-5), (np.float64, 1e-10)], ids=['c64', 'c128'])
