@@ -739,29 +739,29 @@ static bool narrow_gates(const std::vector<const PendingGate *> &gates, unsigned
     return true;
 }
 
-// Whether the diagonal gates can run as fixed-point phases (entries of modulus
-// at most 1).
-static bool bounded_phases(const std::vector<const PendingGate *> &gates) {
-    for (const PendingGate *g : gates)
-        if (g->diag && !(std::hypot(g->m.v[0], g->m.v[1]) < 1. + 1e-9 &&
-                         std::hypot(g->m.v[6], g->m.v[7]) < 1. + 1e-9))
+// Whether every gate's matrix is unitary (to 1e-6: matrices rounded to single
+// precision pass).  Complex128 tensor stages cut a fused block into digits below
+// the norm of its largest row and phases to fixed point: exact to FP64 for a
+// unitary's rows, all of norm 1, but not for products whose rows differ in norm
+// by many orders.  A stage with another matrix runs on the CUDA cores.
+static bool unitary_gates(const std::vector<const PendingGate *> &gates) {
+    for (const PendingGate *g : gates) {
+        const double *v = g->m.v;  // rows (a, b), (c, d)
+        const double r0 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
+        const double r1 = v[4] * v[4] + v[5] * v[5] + v[6] * v[6] + v[7] * v[7];
+        const double re = v[0] * v[4] + v[1] * v[5] + v[2] * v[6] + v[3] * v[7];
+        const double im = v[1] * v[4] - v[0] * v[5] + v[3] * v[6] - v[2] * v[7];
+        if (!(std::fabs(r0 - 1.) < 1e-6 && std::fabs(r1 - 1.) < 1e-6 && std::fabs(re) < 1e-6 &&
+              std::fabs(im) < 1e-6))
             return false;
-    return true;
-}
-
-// Digits can only be cut from finite matrices; a stage with another one runs
-// on the CUDA cores.
-static bool finite_gates(const std::vector<const PendingGate *> &gates) {
-    for (const PendingGate *g : gates)
-        for (double v : g->m.v)
-            if (!(std::fabs(v) < 1e100)) return false;
+    }
     return true;
 }
 
 static void run_tstage(Device &d, States *s, const TileLanes &tl,
                        const std::vector<const PendingGate *> &gates) {
     const int n = s->n_lanes;
-    const TcOps ops = tc_ops(tc_blocks(gates, tl), s->prec == kFP32 || bounded_phases(gates));
+    const TcOps ops = tc_ops(tc_blocks(gates, tl), true);
     if (!d.h_bring) {
         QG_CUDA(cudaMallocHost(&d.h_bring, Device::kBRingBytes));
         QG_CUDA(cudaMalloc(&d.d_bring, Device::kBRingBytes));
@@ -833,7 +833,7 @@ static void run_stage(Device &d, States *s, unsigned long long S,
     // Valid shapes: 32..512 threads (256 with 5 register lanes), 3..5
     // register lanes (complex128 at most 4).
     if (d.tensor_blocks && (m == 12 || (m == 13 && s->prec == kFP32)) && n >= m &&
-        narrow_gates(gates, S) && (s->prec == kFP32 || finite_gates(gates))) {
+        narrow_gates(gates, S) && (s->prec == kFP32 || unitary_gates(gates))) {
         run_tstage(d, s, tl, gates);
         return;
     }

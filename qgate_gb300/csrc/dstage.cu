@@ -23,7 +23,10 @@
 //    excess rounds at 2^-24 of that level);
 //  - the result sum_d L_d 2^(-10 (d - 2)) is formed as a 64-bit integer again.
 // What is left out: digits of V below 2^-52 of the tile's largest component
-// (rounded), of the matrix below 2^-53, and levels d >= 8 (2^-60).  Whole circuits
+// (rounded), of the matrix below 2^-53, and levels d >= 8 (2^-60).  An amplitude far
+// below its tile's largest one so carries an error of the tile's size, as under any
+// gate that mixes the two.  Stages with a matrix that is not unitary do not come
+// here: products of such matrices can have rows of very different norm.  Whole circuits
 // against 64-bit arithmetic (2-norm): random U3 + CX, 26 qubits, 8 layers 7.5e-15
 // (the double-float CUDA-core stages: 4.4e-14), Ising steps 2.6e-14 (3.8e-14), a
 // 25-qubit QFT of a product state 1.2e-14 (1.9e-14).
@@ -618,7 +621,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                 E += sh;
                 unsigned off = PH ? offset : kOffset;
                 if (sh < 3) {
-                    // a tile that shrank (under a singular matrix): scaled up
+                    // a tile that shrank: scaled up
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
                         const unsigned long long V = (join64(v[2 * j], v[2 * j + 1]) - off) << (3 - sh);

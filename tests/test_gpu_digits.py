@@ -111,6 +111,33 @@ def test_matrices_that_are_not_unitary(rt, nat, graph):
     circ.delete()
 
 
+def test_rows_of_very_different_norm_keep_their_precision(rt, nat):
+    """A damping of 1e-12 on one lane between rotations, all in one stage: the
+    damped half is as exact as the other (1e-12 of its norm).  (A later stage of
+    unitary gates alone runs on the tensor cores again, whose digits are cut
+    below the largest component of the whole tile.)"""
+    from qgate_gb300.compiled import CompiledCircuit
+    n = 12
+    rng = np.random.default_rng(n)
+    h = np.array([[1., 1.], [1., -1.]]) / np.sqrt(2.)
+    damp = np.diag([1., 1e-12])
+    gates = [(h, False, q, []) for q in range(n)] + [(damp, False, 5, [])]
+    gates += [(h, False, q, [(q + 1) % n]) for q in range(n) if q != 5]
+    v = rng.normal(size=(1 << n, 2)) @ np.array([1., 1j])
+    v /= np.linalg.norm(v)
+    want = sv.run_ops(n, [('m', m, [t], c) for m, _, t, c in gates], np.complex128, psi=v.copy())
+    circ = CompiledCircuit(np.float64, gates, graph=False)
+    qs = new_state(rt, n, np.float64)
+    qs.set_raw(v)
+    circ.run(qs)
+    got = qs.get_raw()
+    qs.delete()
+    circ.delete()
+    half = (np.arange(1 << n) >> 5 & 1) == 1
+    for part in (half, ~half):
+        assert np.linalg.norm((got - want)[part]) < 1e-12 * np.linalg.norm(want[part])
+
+
 def test_a_nan_stays_in_its_tile_and_ends(rt, nat):
     n = 14
     v = np.full(1 << n, 2. ** -7, np.complex128)
