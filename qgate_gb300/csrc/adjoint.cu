@@ -57,11 +57,36 @@ template <class R> __device__ __forceinline__ R warp_sum(R v) {
     return v;
 }
 
+// Global offset of register j: the sum of e[k] over the set bits k of j.
+template <int RL> __device__ __forceinline__ idx_t reg_offset(const idx_t (&e)[RL], int j) {
+    idx_t o = 0;
+#pragma unroll
+    for (int k = 0; k < RL; ++k)
+        if (j & (1 << k)) o += e[k];
+    return o;
+}
+
+// CTAs per SM the registers leave room for.  complex64 backward stages: five (48
+// registers without spills) against four 20.4 and 20.7 ms for the gradient below,
+// 14.6 and 15.1 ms without checkpoints; six spill (21.2 and 15.1 ms).
 template <class R, int RL, int MODE>
-__global__ void __launch_bounds__(MODE == 1 ? 256 : 512)
+constexpr int kAdjBlocks = MODE == 1 && RL == 3 && sizeof(R) == 4 ? 5 : 0;
+
+// Backward stages read psi and lambda and write lambda (psi too where no
+// checkpoint follows): HBM sets the floor, 60 us for 16 vectors of 20 qubits.  A
+// stage whose register set holds none of the lowest lanes runs from global loads
+// to global stores in registers, without shared memory or its barriers; with
+// several sets the first and the last do so.  Psi is carried only as far as the
+// last gradient where nothing reads it after, and not read without one.  20 qubits,
+// 6 layers, batch 16, a checkpoint every 3 gates: a stage of diagonal rotations
+// 90 us, of RY 97, of CX (lambda alone: 40 us of HBM) 61; 96 to 111 before, when
+// every stage went through shared memory with both states.  What is left is issue
+// (runtime control masks on every register).
+template <class R, int RL, int MODE>
+__global__ void __launch_bounds__(MODE == 1 ? 256 : 512, kAdjBlocks<R, RL, MODE>)
 k_adj_stage(const typename CT<R>::type *psi_src, typename CT<R>::type *psi_dst,
             typename CT<R>::type *lam_all, int store_lam, const __grid_constant__ AdjStageDesc d,
-            const R *__restrict__ mats_all, R *__restrict__ gpart) {
+            const R *__restrict__ mats_all, R *__restrict__ gpart, int slot_stride) {
     typedef typename CT<R>::type C;
     constexpr int NR = 1 << RL;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -72,48 +97,72 @@ k_adj_stage(const typename CT<R>::type *psi_src, typename CT<R>::type *psi_dst,
     const C *psi = psi_src + ((idx_t)b << n);
     C *lam = MODE == 1 ? lam_all + ((idx_t)b << n) : nullptr;
 
+    const unsigned tile = adj_in_registers(d) ? 0u : 1u << m;
     C *sp = (C *)smraw;
-    C *sl = sp + (MODE == 1 ? (1 << m) : 0);
-    AdjOp *sops = (AdjOp *)(sp + ((MODE == 1 ? 2 : 1) << m));
-    long long *sdep = (long long *)(sops + d.nops);
-    SetSlots *sset = (SetSlots *)(sdep + NR);
+    C *sl = sp + (MODE == 1 ? tile : 0u);
+    AdjOp *sops = (AdjOp *)(sp + (MODE == 1 ? 2u : 1u) * tile);
+    SetSlots *sset = (SetSlots *)(sops + d.nops);
     R *smat = (R *)((unsigned char *)sset + adj_sets_bytes(d.nsets));
     R *sgrad = smat + 8 * d.nmats;
 
+    // psi goes nowhere when a checkpoint replaces it next, lambda when no
+    // rotation is left before it
+    const bool keep_psi = MODE == 0 || psi_dst != nullptr, keep_lam = MODE == 1 && store_lam;
+    const bool use_psi = keep_psi || d.last_grad >= 0;
+    const int t = m - RL;
+    const idx_t base = insert_zeros((idx_t)blockIdx.x, d.ins_pos, d.nins);
+    auto thread_offset = [&](int f) {
+        idx_t o = base;
+        for (int k = 0; k < t; ++k)
+            if (tid >> k & 1u) o |= 1LL << d.io_lane[f][k];
+        return o;
+    };
+    auto register_lanes = [&](int f, idx_t (&e)[RL]) {
+#pragma unroll
+        for (int k = 0; k < RL; ++k) e[k] = 1LL << d.io_lane[f][t + k];
+    };
+    const unsigned pt = Swz<R>::f(tid);
+    C a[NR], l[NR];
+    {
+        const idx_t g0 = thread_offset(0);
+        idx_t e[RL];
+        register_lanes(0, e);
+        if (d.direct_in) {
+#pragma unroll
+            for (int j = 0; j < NR; ++j) {
+                const idx_t g = g0 + reg_offset<RL>(e, j);
+                if (MODE == 0 && !psi_src)
+                    a[j] = cmk<C>(g == 0 ? 1. : 0., 0.);  // |0...0>
+                else if (use_psi)
+                    a[j] = psi[g];
+                if (MODE == 1) l[j] = lam[g];
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < NR; ++i) {
+                const unsigned slot = pt ^ Swz<R>::f((unsigned)i << t);
+                const idx_t g = g0 + reg_offset<RL>(e, i);
+                if (MODE == 0 && !psi_src)
+                    sp[slot] = cmk<C>(g == 0 ? 1. : 0., 0.);  // |0...0>
+                else if (use_psi)
+                    cp_async_elem(&sp[slot], &psi[g]);
+                if (MODE == 1) cp_async_elem(&sl[slot], &lam[g]);
+            }
+        }
+    }
     {
         const int4 *src = (const int4 *)d.ops;
         int4 *dst = (int4 *)sops;
         for (int i = tid; i < d.nops; i += T) dst[i] = src[i];
-        if (tid < (unsigned)NR) sdep[tid] = d.dep_hi[tid];
         copy_sets(sset, d.sets, d.nsets, tid, T);
         const R *mats = mats_all + (size_t)b * d.nmats * 8;
         for (int i = tid; i < 8 * d.nmats; i += T) smat[i] = mats[i];
         if (MODE == 1)
             for (int i = tid; i < d.ngrads; i += T) sgrad[i] = 0;
     }
-    const int t = m - RL;
-    const idx_t base = insert_zeros((idx_t)blockIdx.x, d.ins_pos, d.nins);
-    const int lr = d.lowrun < t ? d.lowrun : t;
-    idx_t dt = (idx_t)(tid & ((1u << lr) - 1u));
-    for (int bb = lr; bb < t; ++bb)
-        if (tid & (1u << bb)) dt |= 1LL << d.hi_pos[bb - d.lowrun];
-    const unsigned pt = Swz<R>::f(tid);
-    __syncthreads();
-
-#pragma unroll
-    for (int i = 0; i < NR; ++i) {
-        unsigned slot = pt ^ Swz<R>::f((unsigned)i << t);
-        idx_t g = base | dt | sdep[i];
-        if (MODE == 0 && !psi_src)
-            sp[slot] = cmk<C>(g == 0 ? 1. : 0., 0.);  // |0...0>
-        else
-            cp_async_elem(&sp[slot], &psi[g]);
-        if (MODE == 1) cp_async_elem(&sl[slot], &lam[g]);
-    }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
 
-    C a[NR], l[NR];
     unsigned e0 = 0, P0 = 0;
     unsigned q[RL];
 #pragma unroll
@@ -122,14 +171,17 @@ k_adj_stage(const typename CT<R>::type *psi_src, typename CT<R>::type *psi_dst,
 
     for (int oi = 0; oi < d.nops; ++oi) {
         const AdjOp o = sops[oi];
+        // whether the op has to change psi, lambda
+        const bool on_psi = keep_psi || oi < d.last_grad;
+        const bool on_lam = MODE == 1 && (keep_lam || oi < d.last_grad);
         if (o.kind == kOpTranspose) {
             if (oi > 0) {
                 __syncthreads();
 #pragma unroll
                 for (int j = 0; j < NR; ++j) {
                     unsigned sl_ = reg_slot<RL>(P0, q, j);
-                    sp[sl_] = a[j];
-                    if (MODE == 1) sl[sl_] = l[j];
+                    if (on_psi) sp[sl_] = a[j];
+                    if (on_lam) sl[sl_] = l[j];
                 }
                 __syncthreads();
             }
@@ -138,11 +190,12 @@ k_adj_stage(const typename CT<R>::type *psi_src, typename CT<R>::type *psi_dst,
             e0 = Swz<R>::f(P0);
 #pragma unroll
             for (int k = 0; k < RL; ++k) q[k] = ss.q[k];
+            if (oi == 0 && d.direct_in) continue;
 #pragma unroll
             for (int j = 0; j < NR; ++j) {
                 unsigned sl_ = reg_slot<RL>(P0, q, j);
-                a[j] = sp[sl_];
-                if (MODE == 1) l[j] = sl[sl_];
+                if (on_psi) a[j] = sp[sl_];
+                if (on_lam) l[j] = sl[sl_];
             }
             continue;
         }
@@ -171,59 +224,67 @@ k_adj_stage(const typename CT<R>::type *psi_src, typename CT<R>::type *psi_dst,
             mm.m01 = cmk<C>(mm_[2], mm_[3]);
             mm.m10 = cmk<C>(mm_[4], mm_[5]);
             mm.m11 = cmk<C>(mm_[6], mm_[7]);
-            QG_REG_DISPATCH(reg_gate, o.reg, a, mm, (unsigned)o.jmask);
-            if (MODE == 1) QG_REG_DISPATCH(reg_gate, o.reg, l, mm, (unsigned)o.jmask);
+            if (on_psi) QG_REG_DISPATCH(reg_gate, o.reg, a, mm, (unsigned)o.jmask);
+            if (on_lam) QG_REG_DISPATCH(reg_gate, o.reg, l, mm, (unsigned)o.jmask);
         } else if (o.kind == kOpSwapX) {
-            QG_REG_DISPATCH(reg_swap, o.reg, a, (unsigned)o.jmask);
-            if (MODE == 1) QG_REG_DISPATCH(reg_swap, o.reg, l, (unsigned)o.jmask);
+            if (on_psi) QG_REG_DISPATCH(reg_swap, o.reg, a, (unsigned)o.jmask);
+            if (on_lam) QG_REG_DISPATCH(reg_swap, o.reg, l, (unsigned)o.jmask);
         } else if (o.kind == kOpDiagReg) {
             C d0 = cmk<C>(mm_[0], mm_[1]), d1 = cmk<C>(mm_[6], mm_[7]);
-            QG_REG_DISPATCH(reg_diag, o.reg, a, d0, d1, (unsigned)o.jmask);
-            if (MODE == 1) QG_REG_DISPATCH(reg_diag, o.reg, l, d0, d1, (unsigned)o.jmask);
+            if (on_psi) QG_REG_DISPATCH(reg_diag, o.reg, a, d0, d1, (unsigned)o.jmask);
+            if (on_lam) QG_REG_DISPATCH(reg_diag, o.reg, l, d0, d1, (unsigned)o.jmask);
         } else {  // kOpDiagThread
             C ph = (e0 & o.tbit) ? cmk<C>(mm_[6], mm_[7]) : cmk<C>(mm_[0], mm_[1]);
 #pragma unroll
             for (int j = 0; j < NR; ++j)
                 if ((j & o.jmask) == o.jmask) {
-                    a[j] = cmul(ph, a[j]);
-                    if (MODE == 1) l[j] = cmul(ph, l[j]);
+                    if (on_psi) a[j] = cmul(ph, a[j]);
+                    if (on_lam) l[j] = cmul(ph, l[j]);
                 }
         }
     }
 
-    // psi goes nowhere when a checkpoint replaces it next, lambda when no
-    // rotation is left before it
-    const bool keep_psi = MODE == 0 || psi_dst != nullptr, keep_lam = MODE == 1 && store_lam;
     __syncthreads();
     if (keep_psi || keep_lam) {
-#pragma unroll
-        for (int j = 0; j < NR; ++j) {
-            unsigned sl_ = reg_slot<RL>(P0, q, j);
-            if (keep_psi) sp[sl_] = a[j];
-            if (keep_lam) sl[sl_] = l[j];
-        }
-        __syncthreads();
+        const idx_t g0 = thread_offset(1);
+        idx_t e[RL];
+        register_lanes(1, e);
         C *out = psi_dst + ((idx_t)b << n);
+        if (d.direct_out) {
 #pragma unroll
-        for (int i = 0; i < NR; ++i) {
-            unsigned slot = pt ^ Swz<R>::f((unsigned)i << t);
-            idx_t g = base | dt | sdep[i];
-            if (keep_psi) out[g] = sp[slot];
-            if (keep_lam) lam[g] = sl[slot];
+            for (int j = 0; j < NR; ++j) {
+                const idx_t g = g0 + reg_offset<RL>(e, j);
+                if (keep_psi) out[g] = a[j];
+                if (keep_lam) lam[g] = l[j];
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < NR; ++j) {
+                unsigned sl_ = reg_slot<RL>(P0, q, j);
+                if (keep_psi) sp[sl_] = a[j];
+                if (keep_lam) sl[sl_] = l[j];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < NR; ++i) {
+                const unsigned slot = pt ^ Swz<R>::f((unsigned)i << t);
+                const idx_t g = g0 + reg_offset<RL>(e, i);
+                if (keep_psi) out[g] = sp[slot];
+                if (keep_lam) lam[g] = sl[slot];
+            }
         }
     }
     if (MODE == 1)
         for (int i = tid; i < d.ngrads; i += T)
-            gpart[((idx_t)b * d.ngrads + i) * tiles + blockIdx.x] = sgrad[i];
+            gpart[((idx_t)b * slot_stride + i) * tiles + blockIdx.x] = sgrad[i];
 }
 
-// grad[b * n_params + param[s]] += scale[s] * sum over tiles, FP64.
+// sums[b * nslots + s] = sum over tiles of slot s's partials, FP64.
 template <class R>
-__global__ void k_adj_grad_reduce(const R *__restrict__ partials, int nslots, idx_t tiles,
-                                  const int *__restrict__ param, const double *__restrict__ scale,
-                                  double *__restrict__ grad, int n_params) {
+__global__ void k_adj_grad_reduce(const R *__restrict__ partials, int slot_stride, idx_t tiles,
+                                  double *__restrict__ sums, int nslots) {
     const int s = blockIdx.x, b = blockIdx.y;
-    const R *p = partials + ((idx_t)b * nslots + s) * tiles;
+    const R *p = partials + ((idx_t)b * slot_stride + s) * tiles;
     double acc = 0.;
     for (idx_t i = threadIdx.x; i < tiles; i += blockDim.x) acc += (double)p[i];
     __shared__ double ws[32];
@@ -233,7 +294,7 @@ __global__ void k_adj_grad_reduce(const R *__restrict__ partials, int nslots, id
     if (threadIdx.x == 0) {
         double v = 0.;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += ws[w];
-        if (param[s] >= 0) grad[(idx_t)b * n_params + param[s]] += scale[s] * v;
+        sums[(idx_t)b * nslots + s] = v;
     }
 }
 
@@ -347,12 +408,11 @@ constexpr int kPauliBlocks = 152 * 2;
 
 template <class R, int MODE>
 void adj_dispatch(const void *psi_src, void *psi_dst, void *lam, bool store_lam,
-                  const AdjStageDesc &d, const void *mats, void *gpart, int batch,
+                  const AdjStageDesc &d, const void *mats, void *gpart, int slot_stride, int batch,
                   cudaStream_t stream) {
     typedef typename CT<R>::type C;
-    const int NRmax = 1 << d.rl;
-    size_t smem = ((size_t)sizeof(C) << d.m) * (MODE == 1 ? 2 : 1) + (size_t)d.nops * sizeof(AdjOp) +
-                  sizeof(long long) * NRmax + adj_sets_bytes(d.nsets) +
+    const size_t tile = adj_in_registers(d) ? 0 : (sizeof(C) << d.m) * (MODE == 1 ? 2 : 1);
+    size_t smem = tile + (size_t)d.nops * sizeof(AdjOp) + adj_sets_bytes(d.nsets) +
                   sizeof(R) * (8 * (size_t)d.nmats + (size_t)d.ngrads);
     idx_t tiles = (idx_t)1 << (d.n - d.m);
     int threads = 1 << (d.m - d.rl);
@@ -360,7 +420,8 @@ void adj_dispatch(const void *psi_src, void *psi_dst, void *lam, bool store_lam,
     auto launch = [&](auto kern) {
         QG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         kern<<<grid, threads, smem, stream>>>((const C *)psi_src, (C *)psi_dst, (C *)lam,
-                                              store_lam ? 1 : 0, d, (const R *)mats, (R *)gpart);
+                                              store_lam ? 1 : 0, d, (const R *)mats, (R *)gpart,
+                                              slot_stride);
     };
     switch (d.rl) {
     case 3: launch(k_adj_stage<R, 3, MODE>); break;
@@ -382,9 +443,10 @@ void adj_dispatch(const void *psi_src, void *psi_dst, void *lam, bool store_lam,
 
 void launch_adj_stage(int prec, int mode, const void *psi_src, void *psi_dst, void *lam,
                       bool store_lam, const AdjStageDesc &d, const void *mats,
-                      void *grad_partials, int batch, cudaStream_t stream) {
+                      void *grad_partials, int slot_stride, int batch, cudaStream_t stream) {
     auto run = [&](auto dispatch) {
-        dispatch(psi_src, psi_dst, lam, store_lam, d, mats, grad_partials, batch, stream);
+        dispatch(psi_src, psi_dst, lam, store_lam, d, mats, grad_partials, slot_stride, batch,
+                 stream);
     };
     if (prec == kFP32) {
         if (mode == 0)
@@ -399,18 +461,16 @@ void launch_adj_stage(int prec, int mode, const void *psi_src, void *psi_dst, vo
     }
 }
 
-void launch_adj_grad_reduce(int prec, const void *partials, int batch, int nslots, idx_t tiles,
-                            const int *d_param, const double *d_scale, double *grad,
-                            int n_params, cudaStream_t stream) {
-    if (nslots == 0) return;
-    dim3 grid((unsigned)nslots, (unsigned)batch);
+void launch_adj_grad_reduce(int prec, const void *partials, int batch, int slots, int slot_stride,
+                            idx_t tiles, double *sums, int nslots, cudaStream_t stream) {
+    if (slots == 0) return;
+    dim3 grid((unsigned)slots, (unsigned)batch);
     if (prec == kFP32)
-        k_adj_grad_reduce<float><<<grid, 256, 0, stream>>>((const float *)partials, nslots, tiles,
-                                                           d_param, d_scale, grad, n_params);
+        k_adj_grad_reduce<float><<<grid, 256, 0, stream>>>((const float *)partials, slot_stride,
+                                                           tiles, sums, nslots);
     else
-        k_adj_grad_reduce<double><<<grid, 256, 0, stream>>>((const double *)partials, nslots,
-                                                            tiles, d_param, d_scale, grad,
-                                                            n_params);
+        k_adj_grad_reduce<double><<<grid, 256, 0, stream>>>((const double *)partials, slot_stride,
+                                                            tiles, sums, nslots);
     QG_CUDA(cudaGetLastError());
 }
 

@@ -155,20 +155,12 @@ bool schedule(const std::vector<Op> &ops, const std::vector<int> &idxs, unsigned
     while (lowrun < m && lanes[lowrun] == lowrun) ++lowrun;
     const int t = m - rl;
     memset(&d, 0, sizeof(d));
+    d.last_grad = -1;
     d.n = n;
     d.m = m;
     d.rl = rl;
-    d.lowrun = lowrun;
-    d.nhi = m - lowrun;
-    for (int j = 0; j < d.nhi; ++j) d.hi_pos[j] = lanes[lowrun + j];
     d.nins = m < n ? m : 0;
     for (int j = 0; j < d.nins; ++j) d.ins_pos[j] = lanes[j];
-    for (int i = 0; i < (1 << rl); ++i) {
-        long long off = 0;
-        for (int k = 0; k < rl; ++k)
-            if (i & (1 << k)) off |= 1LL << lanes[t + k];
-        d.dep_hi[i] = off;
-    }
     mat_src.clear();
     grad_op.clear();
     const int ng = (int)idxs.size();
@@ -197,7 +189,8 @@ bool schedule(const std::vector<Op> &ops, const std::vector<int> &idxs, unsigned
         for (int b : RB)
             if ((int)want.size() < rl && std::find(want.begin(), want.end(), b) == want.end())
                 want.push_back(b);
-        for (int b = 0; b < m && (int)want.size() < rl; ++b)
+        // (from the top: the low lanes stay with the threads)
+        for (int b = m - 1; b >= 0 && (int)want.size() < rl; --b)
             if (std::find(want.begin(), want.end(), b) == want.end()) want.push_back(b);
         if (nsets >= kMaxRegSets || d.nops >= kMaxAdjOps) return false;
         d.sets[nsets] = make_set_slots(want.data(), rl, m, sizeof(R) == 4 ? kFP32 : kFP64);
@@ -210,6 +203,7 @@ bool schedule(const std::vector<Op> &ops, const std::vector<int> &idxs, unsigned
         return true;
     };
     if (!emit_set(upcoming(0))) return false;
+    const std::vector<int> first = RB;
     for (int i = 0; i < ng; ++i) {
         const Op &src = ops[idxs[i]];
         auto pos_in = [&](int b) {
@@ -246,6 +240,7 @@ bool schedule(const std::vector<Op> &ops, const std::vector<int> &idxs, unsigned
             mat_src.push_back(idxs[i]);
         }
         if (mode == 1 && src.kind == 1) {
+            d.last_grad = d.nops - 1;
             if ((int)grad_op.size() >= kMaxAdjSlots) return false;
             o.gaxis = (unsigned char)src.axis;
             o.gslot = (unsigned char)grad_op.size();
@@ -254,6 +249,23 @@ bool schedule(const std::vector<Op> &ops, const std::vector<int> &idxs, unsigned
     }
     d.nmats = (int)mat_src.size();
     d.ngrads = (int)grad_op.size();
+    // Where a register set's lanes all lie above the 128-byte line, its layout is
+    // also one of the global loads or stores (thread bits are the tile's other
+    // lanes in ascending order, as in make_set_slots).
+    auto layout = [&](int f, const std::vector<int> &set) {
+        const int line = sizeof(R) == 4 ? 4 : 3;
+        bool direct = lowrun >= line;
+        for (int b : set) direct = direct && b >= line;
+        int at = 0;
+        for (int b = 0; b < m; ++b)
+            if (direct ? std::find(set.begin(), set.end(), b) == set.end() : b < t)
+                d.io_lane[f][at++] = (signed char)lanes[b];
+        for (int k = 0; k < rl; ++k)
+            d.io_lane[f][at++] = (signed char)lanes[direct ? set[k] : t + k];
+        return direct ? 1 : 0;
+    };
+    d.direct_in = layout(0, first);
+    d.direct_out = layout(1, RB);
     return true;
 }
 
@@ -261,7 +273,6 @@ struct Launch {
     AdjStageDesc desc;
     int mode;
     size_t mat_off;    // element offset (in R) of this stage's [batch][nmats][8] table
-    size_t slot_off;   // offset into the param / scale tables
     int ckpt_before;   // backward: restore psi from this checkpoint first (-1: none)
     int ckpt_after;    // forward: save psi to this checkpoint after (-1: none)
 };
@@ -288,7 +299,6 @@ void build_launches(const std::vector<Op> &ops, const std::vector<int> &order, i
             }
             L.mode = mode;
             L.mat_off = mats.size();
-            L.slot_off = slot_param.size();
             L.ckpt_before = -1;
             L.ckpt_after = -1;
             const int nm = (int)mat_src.size();
@@ -585,23 +595,26 @@ static void adjoint_run(int prec, int n, std::vector<Op> &ops, const double *par
         QG_CUDA(cudaMemcpyAsync(dmats, mats.data(), mats.size() * sizeof(R), cudaMemcpyHostToDevice,
                                 st));
         const int nslot = (int)slot_param.size();
-        int *dparam = (int *)alloc(std::max<size_t>(nslot * sizeof(int), 16));
-        double *dscale = (double *)alloc(std::max<size_t>(nslot * sizeof(double), 16));
-        if (nslot) {
-            QG_CUDA(cudaMemcpyAsync(dparam, slot_param.data(), nslot * sizeof(int),
-                                    cudaMemcpyHostToDevice, st));
-            QG_CUDA(cudaMemcpyAsync(dscale, slot_scale.data(), nslot * sizeof(double),
-                                    cudaMemcpyHostToDevice, st));
-        }
-        double *dgrad = G_out ? (double *)alloc(sizeof(double) * batch * std::max(n_params, 1))
+        // Every rotation has a slot.  The slots' sums over the tiles are formed
+        // for many stages at once (one launch where 64 MB hold the partials: a
+        // launch after each of 84 stages took 0.6 of 20.6 ms), and added to their
+        // parameters on the host, as several may share one.
+        double *dsums = G_out ? (double *)alloc(std::max<size_t>(sizeof(double) * batch * nslot, 16))
                               : nullptr;
-        if (dgrad) QG_CUDA(cudaMemsetAsync(dgrad, 0, sizeof(double) * batch * n_params, st));
+        std::vector<double> sums(G_out ? (size_t)batch * nslot : 0);
         int max_grads = 0;
         for (auto &L : launches) max_grads = std::max(max_grads, L.desc.ngrads);
-        const idx_t tiles_max = (idx_t)1 << (n - std::min(n, M_bwd));
-        void *gpart = G_out && max_grads
-                          ? alloc(sizeof(R) * (size_t)batch * max_grads * (size_t)tiles_max)
-                          : nullptr;
+        const idx_t tiles = (idx_t)1 << (n - std::min(n, M_bwd));
+        const size_t slot_bytes = sizeof(R) * (size_t)batch * (size_t)tiles;
+        const int held = (int)std::max<size_t>(
+            max_grads, std::min<size_t>(nslot, ((size_t)64 << 20) / slot_bytes));
+        char *gpart = G_out && max_grads ? (char *)alloc(slot_bytes * held) : nullptr;
+        int slot0 = 0, slots = 0;  // the slots in gpart
+        auto reduce = [&] {
+            launch_adj_grad_reduce(prec, gpart, batch, slots, held, tiles, dsums + slot0, nslot, st);
+            slot0 += slots;
+            slots = 0;
+        };
         const int pb = pauli_sum_blocks();
         double *epart = (double *)alloc(sizeof(double) * (size_t)batch * pb);
         double *dE = (double *)alloc(sizeof(double) * batch);
@@ -635,13 +648,13 @@ static void adjoint_run(int prec, int n, std::vector<Op> &ops, const double *par
                 store_lam = li + 1 < launches.size();
                 if (!store_lam || launches[li + 1].ckpt_before >= 0) dst = nullptr;
             }
+            if (slots + L.desc.ngrads > held) reduce();
             launch_adj_stage(prec, L.mode, src, dst, lam, store_lam, L.desc,
-                             (const R *)dmats + L.mat_off, gpart, batch, st);
+                             (const R *)dmats + L.mat_off,
+                             gpart ? gpart + sizeof(R) * (size_t)tiles * slots : nullptr, held,
+                             batch, st);
             src = dst;
-            if (L.mode == 1 && L.desc.ngrads)
-                launch_adj_grad_reduce(prec, gpart, batch, L.desc.ngrads,
-                                       (idx_t)1 << (n - L.desc.m), dparam + L.slot_off,
-                                       dscale + L.slot_off, dgrad, n_params, st);
+            slots += L.desc.ngrads;
         }
         if (launches.size() == n_fwd) {
             launch_pauli_sum_apply(prec, psi, lam, n, batch, terms.data(), (int)terms.size(), epart,
@@ -649,10 +662,19 @@ static void adjoint_run(int prec, int n, std::vector<Op> &ops, const double *par
             launch_sum_rows(epart, batch, pb, dE, st);
         }
         QG_CUDA(cudaMemcpyAsync(E_out, dE, sizeof(double) * batch, cudaMemcpyDeviceToHost, st));
-        if (G_out)
-            QG_CUDA(cudaMemcpyAsync(G_out, dgrad, sizeof(double) * batch * n_params,
+        if (slots) reduce();
+        if (!sums.empty())
+            QG_CUDA(cudaMemcpyAsync(sums.data(), dsums, sizeof(double) * sums.size(),
                                     cudaMemcpyDeviceToHost, st));
         QG_CUDA(cudaStreamSynchronize(st));
+        if (G_out) {
+            std::fill(G_out, G_out + (size_t)batch * n_params, 0.);
+            for (int b = 0; b < batch; ++b)
+                for (int s = 0; s < nslot; ++s)
+                    if (slot_param[s] >= 0)
+                        G_out[(size_t)b * n_params + slot_param[s]] +=
+                            slot_scale[s] * sums[(size_t)b * nslot + s];
+        }
     } catch (...) {
         cudaStreamSynchronize(st);
         for (void *p : owned) engine_free(p);

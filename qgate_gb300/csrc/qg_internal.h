@@ -265,31 +265,40 @@ constexpr int kMaxAdjSlots = 128;
 
 struct AdjStageDesc {
     int n, m, rl;
-    int lowrun, nhi;
-    int hi_pos[kMaxTileLanes];
     int nins;
     int ins_pos[kMaxTileLanes];
-    long long dep_hi[1 << kMaxRegLanes];
     int nops, nmats, ngrads, nsets;
+    // The first register set is loaded from the states, the last one stored to
+    // them, without shared memory: its lanes leave the lowest ones (whole 128-byte
+    // lines) to the threads.  io_lane: the lanes of the thread bits, then of the
+    // register bits, at the load [0] and the store [1].
+    int direct_in, direct_out;
+    int last_grad;  // the last op with a gradient (-1: none)
+    signed char io_lane[2][kMaxTileLanes];
     SetSlots sets[kMaxRegSets];
     AdjOp ops[kMaxAdjOps];
 };
+// Whether a stage's tile never goes through shared memory.
+__host__ __device__ inline bool adj_in_registers(const AdjStageDesc &d) {
+    return d.direct_in && d.direct_out && d.nsets == 1;
+}
 
 // mode 0: apply ops to psi.  mode 1: for each op, first accumulate the
 // gradient term Im<lam|P1 G|psi> of its slot (if any), then apply the op's
 // (adjoint) matrix to both psi and lam.  psi is read at psi_src (mode 0:
 // nullptr is |0...0>) and written to psi_dst, which may be the same (mode 1:
-// nullptr where it is not needed any more); lam is updated in place, or left as
+// nullptr where it is not needed any more: psi then stops after the last gradient,
+// and is not read where there is none); lam is updated in place, or left as
 // it was without store_lam.  mats: [batch][nmats][8] in the state's precision;
-// grad_partials: [batch][ngrads][tiles] in the state's precision.  States of
-// batch element b start at b * 2^n.
+// grad_partials: [batch][slot_stride][tiles] in the state's precision, of which
+// the stage writes its ngrads first slots.  States of batch element b start at
+// b * 2^n.
 void launch_adj_stage(int prec, int mode, const void *psi_src, void *psi_dst, void *lam,
                       bool store_lam, const AdjStageDesc &d, const void *mats,
-                      void *grad_partials, int batch, cudaStream_t stream);
-// grad[b * n_params + param[s]] += scale[s] * sum_t partials[b][s][t]  (FP64)
-void launch_adj_grad_reduce(int prec, const void *partials, int batch, int nslots, idx_t tiles,
-                            const int *d_param, const double *d_scale, double *grad,
-                            int n_params, cudaStream_t stream);
+                      void *grad_partials, int slot_stride, int batch, cudaStream_t stream);
+// sums[b * nslots + s] = sum_t partials[b][s][t] of `slots` slots  (FP64)
+void launch_adj_grad_reduce(int prec, const void *partials, int batch, int slots, int slot_stride,
+                            idx_t tiles, double *sums, int nslots, cudaStream_t stream);
 
 struct PauliTerm {
     double coef;

@@ -54,3 +54,28 @@ def test_checkpoints_change_nothing(rt, n, every, dtype, bar):
     ef, _ = _run(n, 2, 3, dtype, every, gradient=False)
     assert np.max(np.abs(e - e0)) < bar * n and np.max(np.abs(ef - e0)) < bar * n
     assert np.max(np.abs(g - g0)) < bar
+
+
+@pytest.mark.parametrize('dtype,bar', [(np.float32, 1e-5), (np.float64, 1e-10)], ids=['c64', 'c128'])
+@pytest.mark.parametrize('n', [8, 13])
+def test_a_shared_parameter_gets_the_sum(rt, n, dtype, bar):
+    """One parameter in every rotation: its gradient is the sum of those of a
+    circuit with a parameter each, with targets and controls on the lowest and the
+    highest lanes and stages with and without rotations."""
+    from qgate_gb300 import adjoint
+    one, many = adjoint.ParamCircuit(n), adjoint.ParamCircuit(n)
+    rng = np.random.default_rng(n)
+    for k in range(30):
+        q, c = (int(x) for x in rng.permutation(n)[:2])
+        for circ, p in ((one, 0), (many, k)):
+            (circ.rx, circ.ry, circ.rz)[k % 3](q, p, (c,) if k % 4 == 0 else ())
+            if k % 5 == 0:
+                circ.cx(c, q)
+                circ.cx(q, (q + 1) % n)
+                circ.gate('H', c)
+    h = adjoint.PauliSum.ising_chain(n).add(0.3, [(0, 'Y'), (n - 1, 'Y')]).add(0.2, [(1, 'Y')])
+    for every in (0, 1, 2):
+        e1, g1 = adjoint.expectation_and_gradient(one, np.full((2, 1), 0.37), h, dtype, every)
+        em, gm = adjoint.expectation_and_gradient(many, np.full((2, 30), 0.37), h, dtype, every)
+        assert np.max(np.abs(e1 - em)) < bar * n
+        assert np.max(np.abs(g1[:, 0] - gm.sum(1))) < bar * 30
