@@ -125,7 +125,9 @@ constexpr float kScale = 4096.f, kUnscale = 1.f / 4096.f;
 // holds 32 / H amplitudes of its row; H = 2 halves the registers per thread
 // so that twice the warps fit); PH = the launch has phase ops (without them
 // the kernel keeps the registers of the dense path alone).
-template <int RT, int G, int H, bool PH>
+// MULTI: the launch covers a batch of states and may read them elsewhere than it
+// writes them (one state in place keeps one pointer and no state offset).
+template <int RT, int G, int H, bool PH, bool MULTI>
 __global__ void __launch_bounds__(128 * RT * G * H, 1)
 k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, int tiles,
          long long state_stride, unsigned ops_stride) {
@@ -193,7 +195,8 @@ k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, 
                           ((32u * (wg & 3u)) << 16);
     const unsigned dcol0 = tmem_sh + g * kColsGroup;       // the group's accumulator
     if (tid == 0)
-        bulk_load(smem_u32(Bs), d.bmats + (size_t)blockIdx.y * ops_stride, d.ops_bytes, bb);
+        bulk_load(smem_u32(Bs), MULTI ? d.bmats + (size_t)blockIdx.y * ops_stride : d.bmats,
+                  d.ops_bytes, bb);
 
     // Load layout: row bit b at global lane row_lane[b], amplitude bit k at
     // the lane of e[k] (chosen per stage on the host; lanes 0..3 of the tile
@@ -219,7 +222,7 @@ k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, 
     // flight during the copy-out; the scale is applied after.
     unsigned v[2 * NA];  // floats (bits): this thread's part of row r
     auto load_raw = [&](int tl) {
-        const float2 *gp0 = src + blockIdx.y * state_stride +
+        const float2 *gp0 = (MULTI ? src + blockIdx.y * state_stride : dst) +
                             (insert_zeros((idx_t)tl, d.ins_pos, d.nins) | row_offset());
         gray_walk<NB>(gp0, e, [&](int j, const float2 *p) {
             const float2 x = *p;
@@ -420,7 +423,7 @@ k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, 
             for (int b = 0; b < t; ++b)
                 if (r & (1u << b)) o |= 1LL << d.out_row_lane[b];
             if (H == 2 && hh) o += d.out_e[4];
-            float2 *gp = dst + blockIdx.y * state_stride +
+            float2 *gp = (MULTI ? dst + blockIdx.y * state_stride : dst) +
                          (insert_zeros((idx_t)tl, d.ins_pos, d.nins) | o);
             gray_walk<NB>(gp, d.out_e, [&](int j, float2 *p) {
                 *p = make_float2(__uint_as_float(v[2 * j]) * kUnscale,
@@ -452,7 +455,7 @@ k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, 
             const SetSlots &nat = sset[nb + 1];
             unsigned slot = (unsigned)nat.lo[r & 31u] ^ (unsigned)nat.hi[r >> 5];
             if (H == 2 && hh) slot ^= nat.q[4];
-            float2 *gp = dst + blockIdx.y * state_stride +
+            float2 *gp = (MULTI ? dst + blockIdx.y * state_stride : dst) +
                          (insert_zeros((idx_t)tl, d.ins_pos, d.nins) | row_offset());
             gray_walk<NB>(gp, e, [&](int j, float2 *p) {
                 const int i = gray_index(j);
@@ -546,12 +549,20 @@ void launch_tstage(void *state, const TcStageDesc &d, cudaStream_t stream, bool 
     };
     bool phases = false;  // phase or cross ops
     for (int b = 0; b < d.nblocks; ++b) phases = phases || d.op_kind[b] != 0;
-    if (d.m == 12 && two_per_row)
-        phases ? launch(k_tstage<1, 3, 2, true>, 3, 768) : launch(k_tstage<1, 3, 2, false>, 3, 768);
-    else if (d.m == 12)
-        phases ? launch(k_tstage<1, 4, 1, true>, 4, 512) : launch(k_tstage<1, 4, 1, false>, 4, 512);
-    else
-        phases ? launch(k_tstage<2, 2, 1, true>, 2, 512) : launch(k_tstage<2, 2, 1, false>, 2, 512);
+    if (batch > 1 || (src && src != state)) {
+        if (d.m != 12 || two_per_row || phases)
+            fail(2, "tensor stage: a batch runs dense ops on 12-lane tiles");
+        launch(k_tstage<1, 4, 1, false, true>, 4, 512);
+    } else if (d.m == 12 && two_per_row) {
+        phases ? launch(k_tstage<1, 3, 2, true, false>, 3, 768)
+               : launch(k_tstage<1, 3, 2, false, false>, 3, 768);
+    } else if (d.m == 12) {
+        phases ? launch(k_tstage<1, 4, 1, true, false>, 4, 512)
+               : launch(k_tstage<1, 4, 1, false, false>, 4, 512);
+    } else {
+        phases ? launch(k_tstage<2, 2, 1, true, false>, 2, 512)
+               : launch(k_tstage<2, 2, 1, false, false>, 2, 512);
+    }
     QG_CUDA(cudaGetLastError());
 }
 
