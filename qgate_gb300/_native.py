@@ -167,8 +167,9 @@ def set_fusion_params(prec, tile_lanes, reg_lanes, cost_budget=0):
 
 
 def set_tensor_blocks(on):
-    """Run complex64 stages of 12/13-lane tiles as fused 5-lane blocks on the
-    tensor cores (tcgen05 kind::f16 on split FP16 operands)."""
+    """Run stages of 12-lane tiles (complex64 13 too) as fused 5-lane blocks on
+    the tensor cores (tcgen05 kind::f16 on split FP16 operands; complex128 on
+    digits).  By default: complex64, and complex128 from 21 lanes."""
     call('qg_set_tensor_blocks', 1 if on else 0)
 
 

@@ -241,6 +241,9 @@ struct Device {
     // complex64 stages on 12- or 13-lane tiles as fused 5-lane blocks on the
     // tensor cores (default; 0 selects the register-resident CUDA-core stage).
     bool tensor_blocks = true;
+    // complex128 states of every size on the tensor stages (the setting made by
+    // hand), else those of kDigitLanes and more.
+    bool digits_always = false;
     // Ring of split block operands: pinned host staging and its device copy.
     static constexpr size_t kBRingBytes = 32ull << 20;
     unsigned char *h_bring = nullptr, *d_bring = nullptr;
@@ -758,6 +761,19 @@ static bool unitary_gates(const std::vector<const PendingGate *> &gates) {
     return true;
 }
 
+// Whether a state's stages run on the tensor cores.  complex128: from 21 lanes.
+// Forming a block's digits and a phase table costs the host more than the
+// CUDA-core program, which a circuit that is run once pays in full: 20 lanes, first
+// pass and repeated ones (replayed), random 12 layers 4.1 and 1.15 ms against 3.0
+// and 1.87, QFT 2.3 and 0.88 against 1.3 and 1.1; 17 lanes, QFT 1.9 and 0.51 against
+// 0.64 and 0.54.  Random, 20 layers: 21 lanes 7.1 and 2.5 against 7.0 and 5.1 ms; 26
+// lanes, 12 layers 25.8 and 24.2 against 84.
+constexpr int kDigitLanes = 21;
+static bool tensor_stages_pay(const Device &d, const States *s) {
+    return d.tensor_blocks &&
+           (s->prec == kFP32 || d.digits_always || s->n_lanes >= kDigitLanes);
+}
+
 static void run_tstage(Device &d, States *s, const TileLanes &tl,
                        const std::vector<const PendingGate *> &gates) {
     const int n = s->n_lanes;
@@ -832,7 +848,7 @@ static void run_stage(Device &d, States *s, unsigned long long S,
     const int m = (int)tl.lanes.size();
     // Valid shapes: 32..512 threads (256 with 5 register lanes), 3..5
     // register lanes (complex128 at most 4).
-    if (d.tensor_blocks && (m == 12 || (m == 13 && s->prec == kFP32)) && n >= m &&
+    if (tensor_stages_pay(d, s) && (m == 12 || (m == 13 && s->prec == kFP32)) && n >= m &&
         narrow_gates(gates, S) && (s->prec == kFP32 || unitary_gates(gates))) {
         run_tstage(d, s, tl, gates);
         return;
@@ -965,7 +981,7 @@ static bool lookahead_params(const Device &d, const States *s, int &M, unsigned 
     const int n = s->n_lanes;
     M = std::min(d.tile_lanes[s->prec], kMaxTileLanes);
     const bool tile = M == 12 || (M == 13 && s->prec == kFP32);
-    if (!(d.tensor_blocks && tile && n > M)) return false;
+    if (!(tensor_stages_pay(d, s) && tile && n > M)) return false;
     base = stage_low_lanes(s);
     return true;
 }
@@ -2057,6 +2073,7 @@ int qg_set_fusion(int max_tile_lanes) {
         g_dev.cost_budget[kFP32] = 0;
         g_dev.cost_budget[kFP64] = 0;
         g_dev.tensor_blocks = true;
+        g_dev.digits_always = false;
         g_dev.pipelined = false;
     } else {
         g_dev.tile_lanes[kFP32] = max_tile_lanes;
@@ -2084,6 +2101,7 @@ int qg_set_tensor_blocks(int on) {
     flush_all();
     g_dev.settings_version += 1;  // compiled circuits re-plan
     g_dev.tensor_blocks = on != 0;
+    g_dev.digits_always = on != 0;
     QG_END
 }
 

@@ -16,6 +16,7 @@ pytestmark = pytest.mark.gpu
 @pytest.fixture
 def nat():
     from qgate_gb300 import _native
+    _native.set_tensor_blocks(True)  # at every size
     _native.timing_enable(True)
     _native.timing_read('', reset=True)
     yield _native
@@ -136,6 +137,19 @@ def test_rows_of_very_different_norm_keep_their_precision(rt, nat):
     half = (np.arange(1 << n) >> 5 & 1) == 1
     for part in (half, ~half):
         assert np.linalg.norm((got - want)[part]) < 1e-12 * np.linalg.norm(want[part])
+
+
+@pytest.mark.parametrize('n', [20, 21])
+def test_default_by_size(rt, nat, n):
+    nat.set_fusion(0)  # the defaults
+    rng = np.random.default_rng(n)
+    ops = _u3_cx(rng, n, 1)
+    qs = new_state(rt, n, np.float64)
+    apply_ops(qs, ops)
+    got = qs.get_raw()
+    qs.delete()
+    assert (nat.timing_read('tstage', reset=True)[0] > 0) == (n >= 21)
+    assert np.max(np.abs(got - sv.run_ops(n, ops, np.complex128))) < 1e-12
 
 
 def test_a_nan_stays_in_its_tile_and_ends(rt, nat):
