@@ -763,11 +763,12 @@ static bool unitary_gates(const std::vector<const PendingGate *> &gates) {
 
 // Whether a state's stages run on the tensor cores.  complex128: from 21 lanes.
 // Forming a block's digits and a phase table costs the host more than the
-// CUDA-core program, which a circuit that is run once pays in full: 20 lanes, first
-// pass and repeated ones (replayed), random 12 layers 4.1 and 1.15 ms against 3.0
-// and 1.87, QFT 2.3 and 0.88 against 1.3 and 1.1; 17 lanes, QFT 1.9 and 0.51 against
-// 0.64 and 0.54.  Random, 20 layers: 21 lanes 7.1 and 2.5 against 7.0 and 5.1 ms; 26
-// lanes, 12 layers 25.8 and 24.2 against 84.
+// CUDA-core program, which a circuit that is run once pays in full.  First pass and
+// repeated ones (replayed) against the CUDA-core stages, ms: 20 lanes, random 12
+// layers 4.1 and 1.15 against 3.0 and 1.87; 21 lanes, random 4 layers 1.8 and 0.88
+// against 1.6 and 1.4, QFT 1.8 and 1.2 against 2.1 and 2.0, Ising 2.5 and 1.1 against
+// 2.3 and 2.2; 22 lanes 2.0 and 1.1 against 2.3 and 2.1, 2.1 and 1.6 against 3.1 and
+// 3.0, 2.8 and 1.2 against 3.3 and 3.2.
 constexpr int kDigitLanes = 21;
 static bool tensor_stages_pay(const Device &d, const States *s) {
     return d.tensor_blocks &&

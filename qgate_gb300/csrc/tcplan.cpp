@@ -696,15 +696,27 @@ static void tc_phase_table(const TcOp &op, const TileLanes &tl, const std::vecto
     int bit_of[64];
     for (int p = 0; p < 64; ++p) bit_of[p] = -1;
     for (int k = 0; k < u; ++k) bit_of[order[k]] = k;
-    for (unsigned idx = 0; idx < (1u << u); ++idx) {
-        cd ph(1., 0.);
-        for (auto *g : op.gates) {
-            bool on = true;
-            for (int c : g->controls) on = on && (idx >> bit_of[tl.local_of[c]] & 1u);
-            if (!on) continue;
-            ph *= (idx >> bit_of[tl.local_of[g->target]] & 1u) ? cd(g->m.v[6], g->m.v[7])
-                                                               : cd(g->m.v[0], g->m.v[1]);
+    // gate by gate over the entries it changes (a QFT's controlled phases: a quarter;
+    // entry by entry over all gates, a 21-lane complex128 QFT's first pass took 3.2 ms
+    // instead of 1.8)
+    const unsigned all = (1u << u) - 1u;
+    std::vector<cd> table(1u << u, cd(1., 0.));
+    for (auto *g : op.gates) {
+        unsigned on = 0;
+        for (int c : g->controls) on |= 1u << bit_of[tl.local_of[c]];
+        const unsigned target = 1u << bit_of[tl.local_of[g->target]];
+        for (int side = 0; side < 2; ++side) {
+            const cd f(g->m.v[6 * side], g->m.v[6 * side + 1]);
+            if (f == cd(1., 0.)) continue;
+            const unsigned fixed = on | (side ? target : 0u), free = all & ~(on | target);
+            for (unsigned k = free;; k = (k - 1u) & free) {
+                table[fixed | k] *= f;
+                if (k == 0) break;
+            }
         }
+    }
+    for (unsigned idx = 0; idx < (1u << u); ++idx) {
+        const cd ph = table[idx];
         const double part[2] = {ph.real(), ph.imag()};
         if (prec == kFP64) {
             int e[4];
