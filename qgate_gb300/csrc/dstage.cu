@@ -231,7 +231,8 @@ __device__ __forceinline__ void combine_levels(unsigned u2, unsigned u3, unsigne
 }
 
 // (re, im) - offset times the phase p = (x + y 2^-32, z + w 2^-32) 2^-30, rounded;
-// the products of the two low parts are dropped (below a quarter unit).
+// the products of two low words are dropped (each below one unit, a third of one
+// on average).  y and w lie within +-(2^31 - 1), as w is negated here.
 __device__ __forceinline__ void phase_mul(unsigned (&v)[64], int j, unsigned offset, int4 p) {
     const unsigned long long re = join64(v[4 * j], v[4 * j + 1]) - offset;
     const unsigned long long im = join64(v[4 * j + 2], v[4 * j + 3]) - offset;

@@ -723,7 +723,9 @@ static void tc_phase_table(const TcOp &op, const TileLanes &tl, const std::vecto
             for (int p = 0; p < 2; ++p) {
                 const double x = part[p] * 0x1p30, h = std::nearbyint(x);
                 e[2 * p] = (int)h;
-                e[2 * p + 1] = (int)std::min(std::nearbyint((x - h) * 0x1p32), 2147483647.);
+                // both ends clamped: the kernel negates this word too
+                e[2 * p + 1] = (int)std::max(
+                    std::min(std::nearbyint((x - h) * 0x1p32), 2147483647.), -2147483647.);
             }
             memcpy(out + 16 * (size_t)idx, e, sizeof(e));
             continue;
