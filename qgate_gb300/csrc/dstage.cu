@@ -231,7 +231,7 @@ __device__ __forceinline__ void combine_levels(unsigned u2, unsigned u3, unsigne
 }
 
 // (re, im) - offset times the phase p = (x + y 2^-32, z + w 2^-32) 2^-30, rounded;
-// the products of two low words are dropped (each below one unit, a third of one
+// the products of two low words are dropped (each below one unit, a quarter
 // on average).  y and w lie within +-(2^31 - 1), as w is negated here.
 __device__ __forceinline__ void phase_mul(unsigned (&v)[64], int j, unsigned offset, int4 p) {
     const unsigned long long re = join64(v[4 * j], v[4 * j + 1]) - offset;
@@ -330,6 +330,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
             done_sh[g] = 0;
         }
         mbar_init(smem_u32(&bar_end), 1);
+        mbar_fence_init();  // bulk copies and commits arrive through the async proxy
         stop_sh = 0;
         dense_0 = -1;
         for (int b = nb - 1; b >= 0; --b)

@@ -178,13 +178,11 @@ k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, 
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    if (tid < G) {
-        mbar_init(smem_u32(&bar_mma[tid]), 1);
-        abort_sh[tid] = 0;
-    }
+    if (tid < G) abort_sh[tid] = 0;
     if (tid == 0) {
+        for (int i = 0; i < G; ++i) mbar_init(smem_u32(&bar_mma[i]), 1);
         mbar_init(bb, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        mbar_fence_init();  // bulk copies and commits arrive through the async proxy
     }
     rs::copy_sets(sset, d.sets, nb + 2, tid, T);
     tc_fence_before();
