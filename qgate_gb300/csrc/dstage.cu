@@ -54,8 +54,12 @@
 // were the limit), addresses formed bit by bit at every use and FP64 conversions
 // with branches 1.7 ms, 5 KB operand chunks instead of 10 KB 1.2 ms.
 //
-// Every wait is bounded; one that gives up sets g_ds_status, both groups and
-// the issuing warp leave, and the CTA still frees its tensor memory.
+// Every wait is bounded: the mbarrier waits by themselves, the polls of the issuing
+// warp and of the operand thread by a count that starts again whenever a group
+// takes a tile, so that it bounds a wait and not the launch.  One that gives up
+// sets g_ds_status; a group decides as a whole whether it leaves (abort_sh[g],
+// written before its barrier and read after it, by its own threads only), the
+// issuing warp leaves when both have, and the CTA frees its tensor memory.
 #include <algorithm>
 #include <cstdint>
 
@@ -296,7 +300,8 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
     __shared__ unsigned tmem_sh;
     __shared__ unsigned red[2][2][8];
     __shared__ volatile int done_sh[2];
-    __shared__ int abort_sh;
+    __shared__ int abort_sh[2];
+    __shared__ volatile unsigned beat_sh[2];  // tiles taken by each group
     __shared__ volatile int stop_sh;
     __shared__ long long row_off[2][40];
     __shared__ unsigned dense_op[kMaxTcBlocks];  // the dense op after op b, in a circle
@@ -308,9 +313,10 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
         if (tid == 0) atomicOr(&g_ds_status, 4u);
         return;
     }
-    if (tid == 0) abort_sh = *(volatile unsigned *)&g_ds_status != 0u;
+    if (tid == 0) stop_sh = *(volatile unsigned *)&g_ds_status != 0u;
     __syncthreads();
-    if (abort_sh) return;
+    if (stop_sh) return;
+    __syncthreads();
     if (warp == 16) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                          smem_u32(&tmem_sh)),
@@ -328,6 +334,8 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                 mbar_init(smem_u32(&bar_e[g][k]), 1);
             }
             done_sh[g] = 0;
+            abort_sh[g] = 0;
+            beat_sh[g] = 0u;
         }
         mbar_init(smem_u32(&bar_end), 1);
         mbar_fence_init();  // bulk copies and commits arrive through the async proxy
@@ -372,8 +380,13 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
             unsigned loaded[2] = {0u, 0u}, slot[2] = {0u, 0u}, part[2] = {0u, 0u};
             unsigned op[2] = {(unsigned)dense_0, (unsigned)dense_0};
             unsigned par[2] = {1u, 1u};  // the first round's slots are free
+            unsigned beat = 0u;
             for (unsigned idle = 0; idle < (1u << 22); ++idle) {
                 if (stop_sh) break;
+                if (beat_sh[0] + beat_sh[1] != beat) {
+                    beat = beat_sh[0] + beat_sh[1];
+                    idle = 0;
+                }
                 if (idle > 1u) __nanosleep(200);
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
@@ -410,31 +423,37 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                 if ((int)(blockIdx.x + g * gridDim.x) < tiles) active |= 1 << g;
             unsigned slot[2] = {0u, 0u}, par[2] = {0u, 0u}, apar[2] = {0u, 0u};
             unsigned fpar = 1u;  // parity of the free-column waits: the first passes
-            unsigned idle = 0;
+            unsigned idle = 0, beat = 0u;
+            // (one decision for the whole warp at every wait)
+            auto all = [](bool x) { return __all_sync(0xffffffffu, x) != 0; };
             const uint64_t da0 = smem_desc(smem_u32(smraw), 16, 1024, 2);
             const uint64_t db0 = smem_desc(ring0, 2560, 128);
 #pragma unroll 1
             while (active && ok) {
+                if (!all(beat_sh[0] + beat_sh[1] == beat)) {
+                    beat = beat_sh[0] + beat_sh[1];
+                    idle = 0;
+                }
                 if (++idle > (1u << 23)) ok = false;
                 if (idle > 1u) __nanosleep(40);
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
                     if (!(active >> g & 1) || !ok) continue;
-                    if (!mbar_test(smem_u32(&bar_a[g]), apar[g])) continue;
+                    if (!all(mbar_test(smem_u32(&bar_a[g]), apar[g]))) continue;
                     idle = 0;
                     apar[g] ^= 1u;
-                    if (done_sh[g]) {
+                    if (all(done_sh[g] != 0)) {
                         active &= ~(1 << g);
                         continue;
                     }
 #pragma unroll
                     for (unsigned h = 0; h < 2u; ++h) {
-                        if (ok && !mbar_wait(smem_u32(&bar_dfree[h]), fpar)) ok = false;
+                        ok = ok && all(mbar_wait(smem_u32(&bar_dfree[h]), fpar));
                         const unsigned dcol = tmem + h * kHalfCols;
 #pragma unroll
                         for (unsigned kp = 0; kp < 2u; ++kp) {
                             const unsigned k = slot[g];
-                            if (ok && !mbar_wait(smem_u32(&bar_b[g][k]), par[g])) ok = false;
+                            ok = ok && all(mbar_wait(smem_u32(&bar_b[g][k]), par[g]));
                             if (!ok) break;
                             tc_fence_after();
                             // A_i: 128-byte swizzled K-major; B_1..: no
@@ -555,6 +574,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
         bool ok = true;
         if (tl < tiles) load_raw(tl);
         for (; tl < tiles && ok; tl += tstep) {
+            if (lt == 0u) beat_sh[g] = beat_sh[g] + 1u;
             unsigned mx = 0;
 #pragma unroll
             for (int j = 0; j < 32; ++j) mx = max(mx, v[2 * j + 1] & 0x7fffffffu);
@@ -666,7 +686,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                 top = low = 0;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    if (!mbar_wait(smem_u32(&bar_d[g][h]), dpar)) ok = false;
+                    if (ok && !mbar_wait(smem_u32(&bar_d[g][h]), dpar)) ok = false;
                     tc_fence_after();
 #pragma unroll
                     for (int c4 = 0; c4 < 4; ++c4) {
@@ -698,7 +718,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                 if (b < nb) split();
             }
             if (!ok) {
-                abort_sh = 1;
+                abort_sh[g] = 1;
                 atomicOr(&g_ds_status, 2u);
             }
 #pragma unroll
@@ -707,7 +727,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
             // one decision for the whole group (its products are read: the
             // digit buffers are free)
             group_sync(gbar, kGT);
-            if (*(volatile int *)&abort_sh) {
+            if (*(volatile int *)&abort_sh[g]) {
                 ok = false;
                 break;
             }
