@@ -9,18 +9,24 @@
 // using fast routines of matrix multiplication", 2012):
 //
 //  - the tile is held as 64-bit integers V with one exponent per tile; before
-//    a block V is shifted so that |V| < 2^49 and cut into five balanced
-//    radix-2^10 digits a1..a5 (|a| <= 512, a4 in halves, a5 within 256 in
-//    eighths: exact in FP16);
+//    a block V is shifted so that |V| < 0.97 2^49 and cut into five balanced
+//    radix-2^10 digits a1..a5 (|a1| <= 498, |a| <= 512, a4 in halves, a5 within
+//    256 in eighths: exact in FP16);
 //  - the host cuts every entry of the block's matrix, scaled so that its rows
 //    have norm <= 1, into digits b1 (|b1| <= 1024), b2..b5 (|b| <= 512; b5 in
 //    quarters);
 //  - level L_d = sum over i + j = d of A_i B_j, d = 2..7, accumulates in its
-//    own FP32 columns of tensor memory.  The sums are integers: |L_2| <= 2^22
-//    (Cauchy-Schwarz), and one product of the other levels is at most
-//    64 * 512 * 512 = 2^24, so FP32 holds them exactly (a level's sum of
-//    several products stays below 2^24 but for adversarial inputs, whose
-//    excess rounds at 2^-24 of that level);
+//    own FP32 columns of tensor memory, A_2 B_2 in a seventh set.  The sums of
+//    d <= 4 are integers that FP32 holds exactly, whatever the tile: of 64 terms
+//    each, with ||B_1|| <= 2^10 + 4 (2-norm of a column), |A_1 B_1| <= 2^22 and
+//    |A_2 B_2| <= 2^24; |A_1 B_j + A_j B_1| <= 498 |B_j|_1 + 2^12 (2^10 + 4), j = 2, 3,
+//    stays below 2^24 where B_2's and B_3's columns have 1-norms of at most 3/4 of
+//    their largest 2^15 (a block of random entries has about 2^14).  The host
+//    finds the ops where they are larger (op_low): before those V is shifted one
+//    bit further, |a1| <= 249.  (With one set per level, a Hadamard block with a
+//    phase on a tile of equal amplitudes, whose digits all add up, went past 2^24
+//    at level 4 in one of ten cases, now and then at level 3: errors up to 4.9e-10.)
+//    L_5 may pass 2^24, and then rounds at 2^-52 of the row's norm;
 //  - the result sum_d L_d 2^(-10 (d - 2)) is formed as a 64-bit integer again.
 // What is left out: digits of V below 2^-52 of the tile's largest component
 // (rounded), of the matrix below 2^-53, and levels d >= 8 (2^-60).  An amplitude far
@@ -37,7 +43,7 @@
 // Data path.  Two groups of 256 threads (two threads per tile row, 16
 // amplitudes each) work on a tile each; warp 16 issues the products of both, warp
 // 17 streams the blocks' operands.  The products of a block run in two halves
-// of 16 outputs (6 levels x 32 columns each): while the tensor core works on
+// of 16 outputs (7 sets x 32 columns each): while the tensor core works on
 // one half, the threads read the other back, and while one group cuts its
 // tile into digits the other's products run.  Operands arrive in chunks of
 // 10 KB (one half, two K-steps of 16) through a ring of three chunks per group.
@@ -84,7 +90,7 @@ constexpr unsigned kGT = 256u;                       // threads per group
 // launch gives 96 registers a thread (61440 in all); the issuing warpgroup
 // returns 64 of its own, so that the groups hold 112: 512 x 112 + 128 x 32.
 constexpr unsigned kThreads = 2u * kGT + 128u;
-constexpr unsigned kLevelCols = 32u, kHalfCols = 6u * kLevelCols;
+constexpr unsigned kLevelCols = 32u, kHalfCols = 7u * kLevelCols;
 
 // Balanced digits: adding 512 to each of the five (256 to the last) makes them
 // unsigned fields.
@@ -209,8 +215,8 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
     return r;
 }
 
-// kOffset + sum_d L_d 2^(34 - 10 (d - 2)) of the six levels, |sum| < 2^57.
-// L_3..L_5 (up to 2^24) become integers by conversion; L_2 and, summed in FP32
+// kOffset + sum_d L_d 2^(34 - 10 (d - 2)) of the six levels, |sum| < 2^57; u4b is
+// A_2 B_2.  L_3..L_5 become integers by conversion; L_2 and, summed in FP32
 // first (their rounding lies 2^-24 below L_6), L_6 and L_7 by the 1.5 * 2^23
 // addition, whose bits 0x4B400000 stay in the low word (kOffset; it makes that
 // word positive, so no sign is extended) and are taken out of the high word by
@@ -218,11 +224,11 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
 // bits is one instruction off the integer pipe, which bounds the kernel's
 // arithmetic, where shifts and adds of 64 bits are four on it.
 __device__ __forceinline__ void combine_levels(unsigned u2, unsigned u3, unsigned u4, unsigned u5,
-                                               unsigned u6, unsigned u7, int m14, int m24,
-                                               unsigned &lo, unsigned &hi) {
+                                               unsigned u6, unsigned u7, unsigned u4b, int m14,
+                                               int m24, unsigned &lo, unsigned &hi) {
     constexpr float kMagic = 12582912.f;  // bits 0x4B400000
     const int i3 = __float2int_rn(__uint_as_float(u3));
-    const int i4 = __float2int_rn(__uint_as_float(u4));
+    const int i4 = __float2int_rn(__uint_as_float(u4)) + __float2int_rn(__uint_as_float(u4b));
     const unsigned b2 = __float_as_uint(__fadd_rn(__uint_as_float(u2), kMagic));
     const float g = __fmaf_rn(__uint_as_float(u7), 0x1p-10f, __uint_as_float(u6));
     const unsigned t = (unsigned)__float2int_rn(__uint_as_float(u5) * 16.f) +
@@ -459,7 +465,8 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                             // A_i: 128-byte swizzled K-major; B_1..: no
                             // swizzle, 160 rows, 8-row groups 128 bytes and
                             // 8-element K-groups 2560 bytes apart.  Level
-                            // i + j: columns 32 (i + j - 2).
+                            // i + j: columns 32 (i + j - 2); A_2 B_2: columns
+                            // 192 and up.
 #pragma unroll
                             for (unsigned q = 0; q < 2u; ++q) {
                                 const unsigned ks = 2u * kp + q;
@@ -471,15 +478,20 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                                 constexpr uint64_t kNext = kSlice >> 4;
                                 mma_f16_lane(dcol, da, db, ks > 0u ? 1u : 0u, idesc_f16(128, 160),
                                              lane);
+                                constexpr uint64_t kB = 512u >> 4;  // 32 rows of B
+                                mma_f16_lane(dcol + 32u, da + kNext, db, 1u, idesc_f16(128, 32),
+                                             lane);
+                                mma_f16_lane(dcol + 192u, da + kNext, db + kB, ks > 0u ? 1u : 0u,
+                                             idesc_f16(128, 32), lane);
                                 if (ks == 0u) {
                                     // level 7 is first written here
-                                    mma_f16_lane(dcol + 32u, da + kNext, db, 1u,
-                                                 idesc_f16(128, 128), lane);
-                                    mma_f16_lane(dcol + 160u, da + kNext, db + (2048u >> 4), 0u,
+                                    mma_f16_lane(dcol + 96u, da + kNext, db + 2 * kB, 1u,
+                                                 idesc_f16(128, 64), lane);
+                                    mma_f16_lane(dcol + 160u, da + kNext, db + 4 * kB, 0u,
                                                  idesc_f16(128, 32), lane);
                                 } else {
-                                    mma_f16_lane(dcol + 32u, da + kNext, db, 1u,
-                                                 idesc_f16(128, 160), lane);
+                                    mma_f16_lane(dcol + 96u, da + kNext, db + 2 * kB, 1u,
+                                                 idesc_f16(128, 96), lane);
                                 }
                                 mma_f16_lane(dcol + 64u, da + 2 * kNext, db, 1u,
                                              idesc_f16(128, 128), lane);
@@ -595,7 +607,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
             }
             // the exponent of the largest component, one more when its
             // mantissa lies within 3 % of the next (the top digit stays below
-            // 512 with its carry)
+            // 498 with its carry)
             const int emax = (int)((mx + 0x8000u) >> 20);
             int E = emax - 1071;  // value = V * 2^E
             if (tl + tstep < tiles) {
@@ -638,8 +650,8 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
             // The integers' digits for dense op b.
             auto split = [&]() {
                 const unsigned most = group_max((unsigned)max(top, ~low));
-                // V 2^-sh below 0.97 * 2^49
-                int sh = 15 - __clz((int)(most + (most >> 5) + 1u));
+                // V 2^-sh below 0.97 * 2^49 (2^48 for an op_low op)
+                int sh = 15 - __clz((int)(most + (most >> 5) + 1u)) + (int)d.op_low[b];
                 E += sh;
                 unsigned off = PH ? offset : kOffset;
                 if (sh < 3) {
@@ -676,9 +688,11 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                 // the biased integers as well, a bit shorter; for half of them
                 // that measured 4 % faster, for all of them slower, as that
                 // pipe does two operations per cycle and SM.)
+                const int etop = emax + (int)d.op_low[0];
+                E += (int)d.op_low[0];
                 slots_walk(sset[0], r, hh, [&](int j, unsigned slot) {
-                    put_digits(a0 + 4u * slot, biased_from_double(v[4 * j], v[4 * j + 1], emax),
-                               biased_from_double(v[4 * j + 2], v[4 * j + 3], emax), 3, one);
+                    put_digits(a0 + 4u * slot, biased_from_double(v[4 * j], v[4 * j + 1], etop),
+                               biased_from_double(v[4 * j + 2], v[4 * j + 3], etop), 3, one);
                 });
             }
             while (b < nb) {  // the digits of dense op b are in place
@@ -690,9 +704,9 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                     tc_fence_after();
 #pragma unroll
                     for (int c4 = 0; c4 < 4; ++c4) {
-                        unsigned L[6][4];
+                        unsigned L[7][4];
 #pragma unroll
-                        for (int l = 0; l < 6; ++l)
+                        for (int l = 0; l < 7; ++l)
                             tmem_ld_x4(tcol + (unsigned)h * kHalfCols + (unsigned)l * kLevelCols +
                                            4u * (unsigned)c4,
                                        L[l]);
@@ -701,7 +715,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                         for (int k = 0; k < 4; ++k) {
                             const int at = 4 * (2 * c4 + (k >> 1) + 8 * h) + 2 * (k & 1);
                             combine_levels(L[0][k], L[1][k], L[2][k], L[3][k], L[4][k], L[5][k],
-                                           m14, m24, v[at], v[at + 1]);
+                                           L[6][k], m14, m24, v[at], v[at + 1]);
                             top = max(top, (int)v[at + 1]);
                             low = min(low, (int)v[at + 1]);
                         }

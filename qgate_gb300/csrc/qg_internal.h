@@ -193,6 +193,7 @@ struct TcStageDesc {
     unsigned op_off[kMaxTcBlocks];        // byte offset of op b's operands
     unsigned char op_kind[kMaxTcBlocks];  // 0: dense block, 1: phase table, 2: cross
     short op_exp[kMaxTcBlocks];           // complex128: op b's matrix is its digits * 2^op_exp
+    unsigned char op_low[kMaxTcBlocks];   // complex128: 1 where op b's digits need smaller inputs
     const unsigned char *bmats;
     SetSlots sets[kMaxTcBlocks + 2];
 };

@@ -305,8 +305,10 @@ static void tc_operand(const std::complex<double> *U, unsigned short *bh, unsign
 // returned: 0 for a unitary), each entry cut into kDigits balanced radix-2^10
 // digits, b1 = rint(x 2^10) and every next one rint of 2^10 times the rest
 // (exact in FP64; the last to quarters), in the chunks described at
-// kDigitOpBytes.
-static int tc_operand_digits(const std::complex<double> *U, unsigned short *out) {
+// kDigitOpBytes.  low: whether the 1-norm of some column of b2 or b3 passes
+// 3/4 of its largest, 64 * 512 (the stage's sums then need smaller inputs).
+static int tc_operand_digits(const std::complex<double> *U, unsigned short *out, bool *low) {
+    *low = false;
     double norm2 = 0.;
     for (int o = 0; o < 32; ++o) {
         double row = 0.;
@@ -326,7 +328,8 @@ static int tc_operand_digits(const std::complex<double> *U, unsigned short *out)
         for (int b = -4096; b <= 4096; ++b) t[b + 4096] = f16_bits(0.25f * (float)b);
         return t;
     }();
-    for (int o = 0; o < 32; ++o)
+    for (int o = 0; o < 32; ++o) {
+        int sum[kDigits] = {0};  // four times the columns' 1-norms
         for (int i = 0; i < 32; ++i)
             for (int part = 0; part < 2; ++part) {
                 // (row, column) of D = A B are (k, n): re at (2i, 2o) and
@@ -343,6 +346,7 @@ static int tc_operand_digits(const std::complex<double> *U, unsigned short *out)
                     const double b = (x + c) - c;
                     x = (x - b) * 1024.;
                     const int v = (int)(4. * b);
+                    sum[j] += v < 0 ? -v : v;
                     if (part == 0) {
                         p[0] = p[9] = f16[4096 + v];
                     } else {
@@ -351,6 +355,8 @@ static int tc_operand_digits(const std::complex<double> *U, unsigned short *out)
                     }
                 }
             }
+        *low = *low || std::max(sum[1], sum[2]) > 4 * 24576;
+    }
     return e;
 }
 
@@ -980,7 +986,9 @@ static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops,
         tc_block_matrix(op.gates, tl, lay, U);
         unsigned short *o = (unsigned short *)(buf + desc.op_off[b]);
         if (prec == kFP64) {
-            desc.op_exp[b] = (short)tc_operand_digits(U, o);
+            bool low;
+            desc.op_exp[b] = (short)tc_operand_digits(U, o, &low);
+            desc.op_low[b] = low ? 1 : 0;
         } else {
             tc_compensate(U);
             tc_operand(U, o, o + 64 * 64);
