@@ -247,6 +247,11 @@ struct Device {
     // Ring of split block operands: pinned host staging and its device copy.
     static constexpr size_t kBRingBytes = 32ull << 20;
     unsigned char *h_bring = nullptr, *d_bring = nullptr;
+    // Marked tiles of a complex128 tensor stage (up to kMarkLanes lanes), one
+    // stage's at a time on the engine's stream; the list is allocated when first
+    // needed.
+    static constexpr int kMarkLanes = 34;
+    TileMarks marks = {nullptr, nullptr};
     // Pinned staging of a batch's programs (grown on demand; reused by the
     // next batch, which starts after this one's results are read).
     unsigned char *h_batch = nullptr;
@@ -300,6 +305,8 @@ static void device_init(int device_id, long long limit) {
     QG_CUDA(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking));
     QG_CUDA(cudaMalloc(&d.d_partials, sizeof(double) * (reduce_partials() + 8)));
     QG_CUDA(cudaMallocHost(&d.h_result, sizeof(double) * 16));
+    QG_CUDA(cudaMalloc(&d.marks.count, 2 * sizeof(unsigned)));
+    QG_CUDA(cudaMemset(d.marks.count, 0, 2 * sizeof(unsigned)));
     for (int i = 0; i < 2; ++i) {
         QG_CUDA(cudaMallocHost(&d.h_stage[i], Device::kStageBytes));
         QG_CUDA(cudaEventCreateWithFlags(&d.ev[i], cudaEventDisableTiming));
@@ -772,7 +779,42 @@ static bool unitary_gates(const std::vector<const PendingGate *> &gates) {
 constexpr int kDigitLanes = 21;
 static bool tensor_stages_pay(const Device &d, const States *s) {
     return d.tensor_blocks &&
-           (s->prec == kFP32 || d.digits_always || s->n_lanes >= kDigitLanes);
+           (s->prec == kFP32 ||
+            ((d.digits_always || s->n_lanes >= kDigitLanes) &&
+             s->n_lanes <= Device::kMarkLanes));
+}
+
+// Whether a complex128 stage keeps its precision on the tensor cores: unitary
+// gates, and one at least that mixes amplitudes (the digits cut below the largest
+// amplitude of a tile, so that permutations would lose what they only move) or
+// none but diagonal ones (which run in FP64).
+static bool digit_stage(const std::vector<const PendingGate *> &gates) {
+    bool mixes = false, diagonal = true;
+    for (const PendingGate *g : gates) {
+        const double *v = g->m.v;
+        mixes = mixes || ((v[0] != 0. || v[1] != 0. || v[6] != 0. || v[7] != 0.) &&
+                          (v[2] != 0. || v[3] != 0. || v[4] != 0. || v[5] != 0.));
+        diagonal = diagonal && g->diag;
+    }
+    return (mixes || diagonal) && unitary_gates(gates);
+}
+
+static void pack_double_float(RStageDesc<double> &desc);
+
+// The register programs of a complex128 tensor launch's gates, for the tiles it
+// marks (several where one descriptor does not hold them).
+static void marked_programs(const Device &d, int n, const TileLanes &tl,
+                            const std::vector<const PendingGate *> &gates,
+                            std::vector<RStageDesc<double>> &out) {
+    out.emplace_back();
+    if (schedule_rstage(gates, tl, n, std::max(3, std::min(d.reg_lanes[kFP64], 4)), out.back())) {
+        pack_double_float(out.back());
+        return;
+    }
+    out.pop_back();
+    const size_t h = gates.size() / 2;
+    marked_programs(d, n, tl, {gates.begin(), gates.begin() + h}, out);
+    marked_programs(d, n, tl, {gates.begin() + h, gates.end()}, out);
 }
 
 static void run_tstage(Device &d, States *s, const TileLanes &tl,
@@ -784,10 +826,22 @@ static void run_tstage(Device &d, States *s, const TileLanes &tl,
         QG_CUDA(cudaMalloc(&d.d_bring, Device::kBRingBytes));
         d.bring_off = 0;
     }
+    if (s->prec == kFP64 && !d.marks.tile)
+        QG_CUDA(cudaMalloc(&d.marks.tile, sizeof(unsigned) << (Device::kMarkLanes - 12)));
     for (size_t b0 = 0; b0 < ops.size();) {
         const int nb = tc_ops_per_launch(ops, b0, s->prec);
         size_t bytes = 0;
         for (int b = 0; b < nb; ++b) bytes += tc_op_bytes(ops[b0 + b], s->prec);
+        const bool phases_only = nb == 1 && ops[b0].phase;
+        const size_t op_bytes = bytes;
+        std::vector<RStageDesc<double>> marked;
+        if (s->prec == kFP64 && !phases_only) {
+            std::vector<const PendingGate *> of;
+            for (int b = 0; b < nb; ++b)
+                of.insert(of.end(), ops[b0 + b].gates.begin(), ops[b0 + b].gates.end());
+            marked_programs(d, n, tl, of, marked);
+            for (auto &p : marked) bytes += rstage_bytes(p);  // (multiples of 16)
+        }
         unsigned char *hb, *db;
         if (d.capturing) {
             // operands a captured graph re-reads: chunks owned by the circuit
@@ -815,15 +869,46 @@ static void run_tstage(Device &d, States *s, const TileLanes &tl,
             d.bring_off += bytes;
         }
         static TcStageDesc desc;
-        tc_plan_launch(tl, n, ops, b0, nb, desc, hb, s->prec);
-        desc.bmats = db;
-        QG_CUDA(cudaMemcpyAsync(db, hb, bytes, cudaMemcpyHostToDevice, d.stream));
-        timed(d, "tstage", [&] {
-            if (s->prec == kFP64)
-                launch_dstage(s->d, desc, d.stream);
-            else
-                launch_tstage(s->d, desc, d.stream, d.pipelined);
-        });
+        if (s->prec == kFP64 && phases_only) {
+            // diagonal gates alone
+            std::vector<int> positions, lanes;
+            for (size_t p = 0; p < tl.lanes.size(); ++p)
+                if (ops[b0].lanes >> p & 1u) {
+                    positions.push_back((int)p);
+                    lanes.push_back(tl.lanes[p]);
+                }
+            tc_phase_values(ops[b0], tl, positions, (std::complex<double> *)hb);
+            QG_CUDA(cudaMemcpyAsync(db, hb, bytes, cudaMemcpyHostToDevice, d.stream));
+            timed(d, "phase", [&] {
+                launch_phase_f64(s->d, n, lanes.data(), (int)lanes.size(), db, d.stream);
+            });
+        } else {
+            tc_plan_launch(tl, n, ops, b0, nb, desc, hb, s->prec);
+            desc.bmats = db;
+            std::vector<size_t> at;
+            for (size_t k = 0, off = op_bytes; k < marked.size(); ++k) {
+                memcpy(hb + off, &marked[k], rstage_bytes(marked[k]));
+                at.push_back(off);
+                off += rstage_bytes(marked[k]);
+            }
+            QG_CUDA(cudaMemcpyAsync(db, hb, bytes, cudaMemcpyHostToDevice, d.stream));
+            timed(d, "tstage", [&] {
+                if (s->prec == kFP64)
+                    launch_dstage(s->d, desc, d.marks, d.stream);
+                else
+                    launch_tstage(s->d, desc, d.stream, d.pipelined);
+            });
+            try {
+                for (size_t k = 0; k < marked.size(); ++k)
+                    timed(d, "marked", [&] {
+                        launch_rstage_marked(s->d, marked[k], db + at[k], d.marks,
+                                             k + 1 < marked.size(), d.stream);
+                    });
+            } catch (...) {
+                cudaMemsetAsync(d.marks.count, 0, 2 * sizeof(unsigned), d.stream);
+                throw;
+            }
+        }
         d.n_passes += 1;
         d.n_bytes += 2 * ((long long)1 << n) * (long long)complex_size(s->prec);
         b0 += nb;
@@ -850,7 +935,7 @@ static void run_stage(Device &d, States *s, unsigned long long S,
     // Valid shapes: 32..512 threads (256 with 5 register lanes), 3..5
     // register lanes (complex128 at most 4).
     if (tensor_stages_pay(d, s) && (m == 12 || (m == 13 && s->prec == kFP32)) && n >= m &&
-        narrow_gates(gates, S) && (s->prec == kFP32 || unitary_gates(gates))) {
+        narrow_gates(gates, S) && (s->prec == kFP32 || digit_stage(gates))) {
         run_tstage(d, s, tl, gates);
         return;
     }

@@ -25,17 +25,28 @@
 //    finds the ops where they are larger (op_low): before those V is shifted one
 //    bit further, |a1| <= 249.  (With one set per level, a Hadamard block with a
 //    phase on a tile of equal amplitudes, whose digits all add up, went past 2^24
-//    at level 4 in one of ten cases, now and then at level 3: errors up to 4.9e-10.)
+//    at level 4, for some phases at level 3 too: errors up to 4.9e-10.)
 //    L_5 may pass 2^24, and then rounds at 2^-52 of the row's norm;
 //  - the result sum_d L_d 2^(-10 (d - 2)) is formed as a 64-bit integer again.
 // What is left out: digits of V below 2^-52 of the tile's largest component
-// (rounded), of the matrix below 2^-53, and levels d >= 8 (2^-60).  An amplitude far
-// below its tile's largest one so carries an error of the tile's size, as under any
-// gate that mixes the two.  Stages with a matrix that is not unitary do not come
-// here: products of such matrices can have rows of very different norm.  Whole circuits
-// against 64-bit arithmetic (2-norm): random U3 + CX, 26 qubits, 8 layers 7.5e-15
-// (the double-float CUDA-core stages: 4.4e-14), Ising steps 2.6e-14 (3.8e-14), a
-// 25-qubit QFT of a product state 1.2e-14 (1.9e-14).
+// (rounded), of the matrix below 2^-53, and levels d >= 8 (2^-60).  These are errors of
+// the size of the tile's largest amplitude, where double-float arithmetic errs by the
+// size of what a gate combines.  So a tile is stored only if its smallest
+// amplitude lies within 2^16 of the largest that its last block read, and is right
+// to 2^-35 of each amplitude then.  Any other tile (products of small rotations, exact
+// zeros, which may stand for less than a digit, rare outcomes beside common ones)
+// is left as it was and marked, and the same gates run on it on the CUDA cores
+// (k_rstage_marked).  16: mixed states hold next to no such tile (random U3 + CX, 22
+// lanes, from the third pass on: none of 10^4; with 13, one in 10^3), while a QFT
+// of a product state has them in half of its passes.  Finding them costs nothing
+// that can be measured; a launch that finds none takes 5 us (k_rstage_marked).
+// Stages with a matrix that is not unitary do not come here (products of such
+// matrices can have rows of very different norm), nor do those without a gate
+// that mixes amplitudes: diagonal ones run as one FP64 table (k_phase_f64),
+// permutations on the CUDA cores.
+// Whole circuits against 64-bit arithmetic (2-norm): random U3 + CX, 26 qubits, 12
+// layers 8.2e-15 (the double-float CUDA-core stages: 5.2e-14), a 25-qubit QFT of
+// a product state 5.9e-15 (2.5e-14).
 //
 // Diagonal gates of one tile run as phase ops (see phase_mul): a table of 64-bit
 // fixed-point phases multiplied into V.
@@ -49,9 +60,9 @@
 // 10 KB (one half, two K-steps of 16) through a ring of three chunks per group.
 //
 // Bound: shared memory, then the groups' chain of phases.  Per tile and block the
-// tensor core reads 160 KB of A and 156 KB of B, 40 KB of operands arrive and the
-// threads write 80 KB of digits: 3400 cycles at 128 B per cycle, beside 2540 of
-// products (19 of the 25 digit pairs, 317 cycles per K-step alone) and about 2400
+// tensor core reads 230 KB of A and 156 KB of B, 40 KB of operands arrive and the
+// threads write 80 KB of digits: 4000 cycles at 128 B per cycle, beside 2800 of
+// products (19 of the 25 digit pairs, 350 cycles per K-step) and about 2400
 // issue slots per scheduler, half of them on the integer pipe.  Measured on the
 // 26-qubit, 12-layer random circuit (3.06 blocks per pass): 17 passes of 1.1 ms,
 // 6600 cycles per tile and block; the CUDA-core stages take 22 passes of 3.6 ms.
@@ -90,6 +101,13 @@ constexpr unsigned kGT = 256u;                       // threads per group
 // launch gives 96 registers a thread (61440 in all); the issuing warpgroup
 // returns 64 of its own, so that the groups hold 112: 512 x 112 + 128 x 32.
 constexpr unsigned kThreads = 2u * kGT + 128u;
+// A tile with an amplitude below 2^-16 of the largest input of its last block is left
+// to the CUDA cores: that input is scaled to 2^49, the block's outputs are 2^4 larger, and
+// these are the high words of 64 bits.
+constexpr unsigned kLeast = 1u << (49 + 4 - 16 - 32);
+// (Only where the largest lies in [2^-45, 2^100): the CUDA cores' FP32 pairs have
+// FP32's exponents, and err by up to 2^-97 below 2^-74.)
+constexpr int kRangeLow = 1023 - 45, kRangeHigh = 1023 + 100;
 constexpr unsigned kLevelCols = 32u, kHalfCols = 7u * kLevelCols;
 
 // Balanced digits: adding 512 to each of the five (256 to the last) makes them
@@ -297,7 +315,8 @@ template <class P, class F> __device__ __forceinline__ void lanes_walk(P *p, con
 // the dense path alone).
 template <bool PH>
 __global__ void __launch_bounds__(kThreads, 1)
-k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles) {
+k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles,
+         const TileMarks marks) {
     extern __shared__ __align__(1024) unsigned char smraw[];
     unsigned char *ring = smraw + 2 * kGroupA;                 // [group][kRing] chunks
     SetSlots *sset = (SetSlots *)(ring + 2 * kRing * kChunk);
@@ -305,6 +324,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
         bar_b[2][kRing], bar_e[2][kRing], bar_end;
     __shared__ unsigned tmem_sh;
     __shared__ unsigned red[2][2][8];
+    __shared__ volatile int wide_sh[2];  // the last tile (+ 1) found wide
     __shared__ volatile int done_sh[2];
     __shared__ int abort_sh[2];
     __shared__ volatile unsigned beat_sh[2];  // tiles taken by each group
@@ -340,6 +360,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                 mbar_init(smem_u32(&bar_e[g][k]), 1);
             }
             done_sh[g] = 0;
+            wide_sh[g] = 0;
             abort_sh[g] = 0;
             beat_sh[g] = 0u;
         }
@@ -591,12 +612,13 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
 #pragma unroll
             for (int j = 0; j < 32; ++j) mx = max(mx, v[2 * j + 1] & 0x7fffffffu);
             mx = group_max(mx);
-            // (an unused tile of zeros stays as it is; components of 2^1018
-            // and more have no room for the digits' constant)
+            // (a tile of zeros, or of subnormals, stays as it is; components of
+            // 2^1018 and more have no room for the digits' constant)
             const bool zero = mx < 0x00100000u, bad = mx >= 0x7fa00000u;
             if (zero || bad) {
                 if (bad) {
-                    // infinities and NaN spread over the tile as NaN
+                    // infinities and NaN spread over the tile as NaN (the CUDA
+                    // cores' FP32 pairs would read them as numbers)
                     uint4 *p0 = tile_base(tl) + row_offset(0);
                     lanes_walk(p0, d.in_e, [&](int, uint4 *p) {
                         *p = make_uint4(0u, 0x7ff80000u, 0u, 0x7ff80000u);
@@ -735,8 +757,19 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                 abort_sh[g] = 1;
                 atomicOr(&g_ds_status, 2u);
             }
+            {
+                // the smallest amplitude (high words; the bits of either part stand
+                // for the larger one, within a factor of two)
+                unsigned least = 0xffffffffu;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) 
+                for (int j = 0; j < 16; ++j) {
+                    const int re = (int)v[4 * j + 1], im = (int)v[4 * j + 3];
+                    least = min(least, (unsigned)((re ^ (re >> 31)) | (im ^ (im >> 31))));
+                }
+                if (least < kLeast && emax >= kRangeLow && emax < kRangeHigh) wide_sh[g] = tl + 1;
+            }
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
                 double_from_fixed(v[2 * j], v[2 * j + 1], PH ? offset : kOffset, E);
             // one decision for the whole group (its products are read: the
             // digit buffers are free)
@@ -744,6 +777,11 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
             if (*(volatile int *)&abort_sh[g]) {
                 ok = false;
                 break;
+            }
+            if (wide_sh[g] == tl + 1) {
+                if (lt == 0u) marks.tile[atomicAdd(&marks.count[0], 1u)] = (unsigned)tl;
+                if (tl + tstep < tiles) load_raw(tl + tstep);
+                continue;
             }
             if (d.direct_out) {
                 // rows in whole 128-byte lines go straight to the state
@@ -787,13 +825,67 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
     }
 }
 
+// Diagonal gates alone: every amplitude times its table entry, in FP64.  1024
+// amplitudes per CTA and step, four per thread; the table's index is the sum of
+// a part by the thread, two by the register and one by the step.  Bound by HBM and
+// the FP64 pipe alike (four multiply-adds per amplitude at two per cycle and SM,
+// 0.23 ms for 25 lanes; HBM 0.16): 0.26 ms, against 0.44 as a phase op of k_dstage.
+struct PhaseLanes {
+    int n;
+    signed char lane[kMaxPhaseLanes];  // ascending
+};
+__global__ void __launch_bounds__(256)
+k_phase_f64(double2 *__restrict__ s, idx_t chunks, const __grid_constant__ PhaseLanes d,
+            const double2 *__restrict__ table) {
+    const unsigned tid = threadIdx.x;
+    unsigned at = 0, r0 = 0, r1 = 0;
+    for (int k = 0; k < d.n; ++k) {
+        const int l = d.lane[k];
+        if (l < 8) at |= (tid >> l & 1u) << k;
+        if (l == 8) r0 = 1u << k;
+        if (l == 9) r1 = 1u << k;
+    }
+    for (idx_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+        unsigned slot = at;
+        for (int k = 0; k < d.n; ++k)
+            if (d.lane[k] >= 10) slot |= (unsigned)(c >> (d.lane[k] - 10) & 1) << k;
+        double2 *p = s + (c << 10) + tid;
+        double2 x[4], f[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            x[u] = p[256 * u];
+            f[u] = __ldg(&table[slot + (u & 1 ? r0 : 0u) + (u & 2 ? r1 : 0u)]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            p[256 * u] = make_double2(x[u].x * f[u].x - x[u].y * f[u].y,
+                                      x[u].x * f[u].y + x[u].y * f[u].x);
+    }
+}
+
 constexpr size_t dstage_smem(int nops) {
     return 2 * (size_t)kGroupA + 2 * (size_t)kRing * kChunk + sizeof(SetSlots) * (size_t)(nops + 2);
 }
 
 }  // namespace
 
-void launch_dstage(void *state, const TcStageDesc &d, cudaStream_t stream) {
+void launch_phase_f64(void *state, int n, const int *lanes, int n_lanes, const void *table,
+                      cudaStream_t stream) {
+    if (n < 10 || n_lanes < 0 || n_lanes > kMaxPhaseLanes)
+        fail(2, "phase pass: bad lane counts %d, %d", n, n_lanes);
+    PhaseLanes d;
+    d.n = n_lanes;
+    for (int k = 0; k < n_lanes; ++k) {
+        if (lanes[k] < 0 || lanes[k] >= n) fail(2, "phase pass: lane %d outside the state", lanes[k]);
+        d.lane[k] = (signed char)lanes[k];
+    }
+    const idx_t chunks = (idx_t)1 << (n - 10);
+    k_phase_f64<<<(unsigned)std::min<idx_t>(chunks, 152 * 8), 256, 0, stream>>>(
+        (double2 *)state, chunks, d, (const double2 *)table);
+    QG_CUDA(cudaGetLastError());
+}
+
+void launch_dstage(void *state, const TcStageDesc &d, const TileMarks &marks, cudaStream_t stream) {
     if (d.m != 12) fail(2, "complex128 tensor stage: tile lanes must be 12 (got %d)", d.m);
     if (d.nblocks < 1 || d.nblocks > kMaxTcBlocks)
         fail(2, "complex128 tensor stage: bad op count %d", d.nblocks);
@@ -817,12 +909,17 @@ void launch_dstage(void *state, const TcStageDesc &d, cudaStream_t stream) {
     QG_CUDA(cudaGetDevice(&dev));
     QG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const size_t smem = dstage_smem(d.nblocks);
-    bool phases = false;
-    for (int b = 0; b < d.nblocks; ++b) phases = phases || d.op_kind[b] != 0;
+    bool phases = false, dense = false;
+    for (int b = 0; b < d.nblocks; ++b) {
+        phases = phases || d.op_kind[b] != 0;
+        dense = dense || d.op_kind[b] == 0;
+    }
+    if (!dense) fail(2, "complex128 tensor stage: no dense op");
     auto launch = [&](auto kern) {
         QG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)dstage_smem(kMaxTcBlocks)));
-        kern<<<(unsigned)std::min(tiles, sms), kThreads, smem, stream>>>((uint4 *)state, d, tiles);
+        kern<<<(unsigned)std::min(tiles, sms), kThreads, smem, stream>>>((uint4 *)state, d, tiles,
+                                                                         marks);
     };
     phases ? launch(k_dstage<true>) : launch(k_dstage<false>);
     QG_CUDA(cudaGetLastError());

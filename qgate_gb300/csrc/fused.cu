@@ -7,6 +7,8 @@
 // one HBM read and one write of the state however many gates it fuses.  The
 // reference has no fusion: every gate is one full-state launch
 // (qgate/simulator/src/DeviceProcPrimitives.cu:198-249).
+#include <algorithm>
+
 #include "qg_device.cuh"
 #include "qg_regstage.cuh"
 
@@ -160,23 +162,26 @@ __device__ __forceinline__ void run_program(typename CT<R>::type *sm, const RegO
 // reads it with broadcast vector loads instead of per-field constant-bank
 // loads.  Load (cp.async, coalesced, swizzled) -> run the program (register
 // gates, diagonal phases, shared-memory transposes) -> store.
-template <class R, int RL, int TL>
-__global__ void __launch_bounds__(1 << TL)
-k_rstage(typename CT<R>::type *__restrict__ s, const __grid_constant__ RStageDesc<R> d) {
+template <class R, int RL, int TL> struct RStageTile {
     typedef typename CT<R>::type C;
     typedef RegOp<R> Op;
-    constexpr int NR = 1 << RL;
-    constexpr int t = TL;                 // thread lanes (tile lanes 0..t-1)
-    constexpr int m = RL + TL;            // tile lanes
-    constexpr unsigned T = 1u << TL;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    C *sm = (C *)smraw;
-    Op *sops = (Op *)(smraw + ((size_t)sizeof(C) << m));
-    long long *sdep = (long long *)(sops + d.nops);
-    SetSlots *sset = (SetSlots *)(sdep + NR);
-    const unsigned tid = threadIdx.x;
+    static constexpr int NR = 1 << RL;
+    static constexpr int t = TL;       // thread lanes (tile lanes 0..t-1)
+    static constexpr int m = RL + TL;  // tile lanes
+    static constexpr unsigned T = 1u << TL;
 
-    {
+    C *sm;
+    Op *sops;
+    long long *sdep;
+    SetSlots *sset;
+
+    // The stage program into shared memory (no barrier after it).
+    __device__ __forceinline__ RStageTile(unsigned char *smraw, const RStageDesc<R> &d) {
+        sm = (C *)smraw;
+        sops = (Op *)(smraw + ((size_t)sizeof(C) << m));
+        sdep = (long long *)(sops + d.nops);
+        sset = (SetSlots *)(sdep + NR);
+        const unsigned tid = threadIdx.x;
         const int4 *src = (const int4 *)d.ops;
         int4 *dst = (int4 *)sops;
         const int nvec = (int)(d.nops * sizeof(Op) / sizeof(int4));
@@ -184,37 +189,75 @@ k_rstage(typename CT<R>::type *__restrict__ s, const __grid_constant__ RStageDes
         if (tid < (unsigned)NR) sdep[tid] = d.dep_hi[tid];
         copy_sets(sset, d.sets, d.nsets, tid, T);
     }
-    const idx_t base = insert_zeros((idx_t)blockIdx.x, d.ins_pos, d.nins);
-    // Global offset of tile element tid (tile lanes 0..t-1); the offsets of
-    // the register-index parts (i << t) are disjoint from it, so element
-    // (tid, i) lives at gp + dep_hi[i].
-    const int lr = d.lowrun < t ? d.lowrun : t;
-    idx_t dt = (idx_t)(tid & ((1u << lr) - 1u));
-    for (int b = lr; b < t; ++b)
-        if (tid & (1u << b)) dt |= 1LL << d.hi_pos[b - d.lowrun];
-    C *const gp = s + (base | dt);
-    const unsigned pt = Swz<R>::f(tid);
-    __syncthreads();
+
+    __device__ __forceinline__ void run(C *s, const RStageDesc<R> &d, idx_t tile) {
+        const unsigned tid = threadIdx.x;
+        const idx_t base = insert_zeros(tile, d.ins_pos, d.nins);
+        // Global offset of tile element tid (tile lanes 0..t-1); the offsets of
+        // the register-index parts (i << t) are disjoint from it, so element
+        // (tid, i) lives at gp + dep_hi[i].
+        const int lr = d.lowrun < t ? d.lowrun : t;
+        idx_t dt = (idx_t)(tid & ((1u << lr) - 1u));
+        for (int b = lr; b < t; ++b)
+            if (tid & (1u << b)) dt |= 1LL << d.hi_pos[b - d.lowrun];
+        C *const gp = s + (base | dt);
+        const unsigned pt = Swz<R>::f(tid);
+        __syncthreads();
 
 #pragma unroll
-    for (int i = 0; i < NR; ++i)
-        cp_async_elem(&sm[pt ^ Swz<R>::f((unsigned)i << t)], gp + sdep[i]);
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncthreads();
+        for (int i = 0; i < NR; ++i)
+            cp_async_elem(&sm[pt ^ Swz<R>::f((unsigned)i << t)], gp + sdep[i]);
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
 
-    typename RegArith<R>::T a[NR];
-    unsigned P0 = 0;
-    unsigned q[RL];
+        typename RegArith<R>::T a[NR];
+        unsigned P0 = 0;
+        unsigned q[RL];
 #pragma unroll
-    for (int k = 0; k < RL; ++k) q[k] = 0;
-    run_program<R, RL, TL>(sm, sops, sset, d.nops, tid, a, P0, q);
+        for (int k = 0; k < RL; ++k) q[k] = 0;
+        run_program<R, RL, TL>(sm, sops, sset, d.nops, tid, a, P0, q);
 
-    __syncthreads();
+        __syncthreads();
 #pragma unroll
-    for (int j = 0; j < NR; ++j) sm[reg_slot<RL>(P0, q, j)] = RegArith<R>::to_tile(a[j]);
-    __syncthreads();
+        for (int j = 0; j < NR; ++j) sm[reg_slot<RL>(P0, q, j)] = RegArith<R>::to_tile(a[j]);
+        __syncthreads();
 #pragma unroll
-    for (int i = 0; i < NR; ++i) gp[sdep[i]] = sm[pt ^ Swz<R>::f((unsigned)i << t)];
+        for (int i = 0; i < NR; ++i) gp[sdep[i]] = sm[pt ^ Swz<R>::f((unsigned)i << t)];
+    }
+};
+
+template <class R, int RL, int TL>
+__global__ void __launch_bounds__(1 << TL)
+k_rstage(typename CT<R>::type *__restrict__ s, const __grid_constant__ RStageDesc<R> d) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    RStageTile<R, RL, TL> tile(smraw, d);
+    tile.run(s, d, (idx_t)blockIdx.x);
+}
+
+// The marked tiles of a complex128 state: those whose digits k_dstage left (see
+// there).  Most launches find few or none, so two CTAs per SM walk the list; the
+// last CTA to end empties it.  (One CTA per four tiles that looks at their marks took
+// 60 us of a 26-qubit state's 16384 tiles, none of them marked.)  The program lies in
+// global memory: as a 23 KB kernel parameter every launch would carry it.  Two
+// resident CTAs of 512 threads need 64 registers, which the loop does not get by itself.
+template <int RL, int TL>
+__global__ void __launch_bounds__(1 << TL, TL == 9 ? 2 : 1)
+k_rstage_marked(double2 *__restrict__ s, const RStageDesc<double> *__restrict__ program,
+                const TileMarks marks, int kept) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const RStageDesc<double> &d = *program;
+    const unsigned count = *(volatile unsigned *)&marks.count[0];
+    if (blockIdx.x < count) {
+        RStageTile<double, RL, TL> tile(smraw, d);
+        for (unsigned i = blockIdx.x; i < count; i += gridDim.x)  // (run begins with a barrier)
+            tile.run(s, d, (idx_t)marks.tile[i]);
+    }
+    if (kept) return;
+    __syncthreads();  // every thread has read the count
+    if (threadIdx.x == 0 && atomicAdd(&marks.count[1], 1u) == gridDim.x - 1u) {
+        marks.count[0] = 0u;
+        marks.count[1] = 0u;
+    }
 }
 
 // Persistent, double-buffered variant: a grid of (SMs x resident CTAs)
@@ -345,6 +388,26 @@ void rstage_dispatch(void *state, const RStageDesc<R> &d, cudaStream_t stream, b
 }
 
 }  // namespace
+
+void launch_rstage_marked(void *state, const RStageDesc<double> &d, const void *program,
+                          const TileMarks &marks, bool kept, cudaStream_t stream) {
+    const size_t smem = ((size_t)1 << d.m) * sizeof(double2) +
+                        (size_t)d.nops * sizeof(RegOp<double>) + sizeof(long long) * (1 << d.rl) +
+                        sizeof(SetSlots) * (size_t)d.nsets;
+    const unsigned ctas = (unsigned)std::min<idx_t>((idx_t)1 << (d.n - d.m), 152 * 2);
+    auto launch = [&](auto kern) {
+        QG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<ctas, 1 << (d.m - d.rl), smem, stream>>>(
+            (double2 *)state, (const RStageDesc<double> *)program, marks, kept ? 1 : 0);
+    };
+    if (d.m == 12 && d.rl == 3)
+        launch(k_rstage_marked<3, 9>);
+    else if (d.m == 12 && d.rl == 4)
+        launch(k_rstage_marked<4, 8>);
+    else
+        fail(2, "marked register stage: unsupported shape m=%d rl=%d", d.m, d.rl);
+    QG_CUDA(cudaGetLastError());
+}
 
 void launch_stage(int prec, void *state, const StageDesc &d, cudaStream_t stream) {
     size_t cs = complex_size(prec);

@@ -211,8 +211,18 @@ void launch_tstage(void *state, const TcStageDesc &d, cudaStream_t stream, bool 
 constexpr int kDigits = 5;
 constexpr unsigned kDigitChunkBytes = 160u * 16u * 2u;
 constexpr unsigned kDigitOpBytes = 8u * kDigitChunkBytes;
-void launch_dstage(void *state, const TcStageDesc &d, cudaStream_t stream);
+// Tiles whose amplitudes the digits would not keep precise (dstage.cu says when) are
+// left as they were and appended to the list, which is empty before the launch.
+struct TileMarks {
+    unsigned *count;  // [2]: tiles in the list, CTAs done with it
+    unsigned *tile;   // as many as a state has tiles
+};
+void launch_dstage(void *state, const TcStageDesc &d, const TileMarks &marks, cudaStream_t stream);
 int dstage_status(bool reset);
+// A complex128 state times table[bits of the index at `lanes`], in FP64.
+constexpr int kMaxPhaseLanes = 12;
+void launch_phase_f64(void *state, int n, const int *lanes, int n_lanes, const void *table,
+                      cudaStream_t stream);
 // Status word of the tensor stage kernels (nonzero: a bounded wait gave up).
 int tstage_status(bool reset);
 
@@ -243,6 +253,14 @@ void launch_rstage_f32(void *state, const RStageDesc<float> &d, cudaStream_t str
                        bool pipelined);
 void launch_rstage_f64(void *state, const RStageDesc<double> &d, cudaStream_t stream,
                        bool pipelined);
+// A complex128 stage on 12-lane tiles, over the marked tiles; empties the list
+// unless it is `kept` for another launch.  program: the device's copy of d, of
+// which rstage_bytes(d) are read.
+inline size_t rstage_bytes(const RStageDesc<double> &d) {
+    return (size_t)((const char *)&d.ops[d.nops] - (const char *)&d);
+}
+void launch_rstage_marked(void *state, const RStageDesc<double> &d, const void *program,
+                          const TileMarks &marks, bool kept, cudaStream_t stream);
 
 // ---------------------------------------------------------------- adjoint
 

@@ -2,6 +2,7 @@
 // engine (adjoint_host.cpp).
 #pragma once
 
+#include <complex>
 #include <utility>
 #include <vector>
 
@@ -80,6 +81,10 @@ struct TcOp {
 };
 typedef std::vector<TcOp> TcOps;
 TcOps tc_ops(const TcBlocks &blocks, bool phases);
+// The entries of a phase op's table, 2^lanes products of its gates' diagonals, in
+// FP64: bit k of the index is the tile position of bit k of `positions`.
+void tc_phase_values(const TcOp &op, const TileLanes &tl, const std::vector<int> &positions,
+                     std::complex<double> *table);
 inline bool tc_dense(const TcOp &op) { return !op.phase && !op.cross; }
 // Operand bytes of an op (complex64; complex128: kDigitOpBytes for a dense op,
 // 16 bytes per entry of a phase table): 16 KB for a dense op (Bh, Bl), 8 bytes per entry of

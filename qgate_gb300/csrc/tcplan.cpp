@@ -689,24 +689,20 @@ int tc_ops_per_launch(const TcOps &ops, size_t b0, int prec) {
     return nb;
 }
 
-// Table of a phase op: entry idx (bit k of idx = tile position order[k]) is
-// the product of the op's diagonal gates' entries at that assignment of
-// their lanes (m00 or m11 of a gate whose controls are all set, else 1),
-// computed in FP64 and rounded to complex64.
-// complex128 tables hold four integers per entry: each part x as rint(x 2^30)
-// and rint of 2^32 times the rest, the real part first.
-static void tc_phase_table(const TcOp &op, const TileLanes &tl, const std::vector<int> &order,
-                           unsigned char *out, int prec) {
+// The product of the op's diagonal gates' entries at every assignment of their
+// lanes (m00 or m11 of a gate whose controls are all set, else 1).
+void tc_phase_values(const TcOp &op, const TileLanes &tl, const std::vector<int> &positions,
+                     std::complex<double> *table) {
     typedef std::complex<double> cd;
-    const int u = (int)order.size();
+    const int u = (int)positions.size();
     int bit_of[64];
     for (int p = 0; p < 64; ++p) bit_of[p] = -1;
-    for (int k = 0; k < u; ++k) bit_of[order[k]] = k;
+    for (int k = 0; k < u; ++k) bit_of[positions[k]] = k;
     // gate by gate over the entries it changes (a QFT's controlled phases: a quarter;
     // entry by entry over all gates, a 21-lane complex128 QFT's first pass took 3.2 ms
     // instead of 1.8)
     const unsigned all = (1u << u) - 1u;
-    std::vector<cd> table(1u << u, cd(1., 0.));
+    std::fill(table, table + (1u << u), cd(1., 0.));
     for (auto *g : op.gates) {
         unsigned on = 0;
         for (int c : g->controls) on |= 1u << bit_of[tl.local_of[c]];
@@ -721,6 +717,17 @@ static void tc_phase_table(const TcOp &op, const TileLanes &tl, const std::vecto
             }
         }
     }
+}
+
+// Table of a phase op: entry idx (bit k of idx = tile position order[k]) in
+// the stage's form: complex64, or for complex128 four integers, each part x as
+// rint(x 2^30) and rint of 2^32 times the rest, the real part first.
+static void tc_phase_table(const TcOp &op, const TileLanes &tl, const std::vector<int> &order,
+                           unsigned char *out, int prec) {
+    typedef std::complex<double> cd;
+    const int u = (int)order.size();
+    std::vector<cd> table(1u << u);
+    tc_phase_values(op, tl, order, table.data());
     for (unsigned idx = 0; idx < (1u << u); ++idx) {
         const cd ph = table[idx];
         const double part[2] = {ph.real(), ph.imag()};
