@@ -10,6 +10,7 @@
 // (qgate/simulator/src/CUDAQubitProcessor.cpp:40-50,
 // qgate/simulator/src/DeviceSum.h:16-23).
 #include "qg_internal.h"
+#include "host_team.h"
 #include "qg_plan.h"
 #include "../../include/qgate_gb300.h"
 
@@ -1229,24 +1230,30 @@ static double read_result(Device &d, double *d_val) {
 // ------------------------------------------------------------ transfers
 
 // Host-side copy between pinned staging and the caller's (pageable) buffer,
-// split over OpenMP threads: one host thread copies 20-40 GB/s, well below
-// what NVLink-C2C delivers into the staging buffers.  A slice of 256 KB is what
-// pays for waking a thread (Grace, medians): 512 KB 15.7 us on one thread, 8.5 on
-// two (10 us on four); 1 MB 33 and 12; 8 MB 437, 196 in slices of 4 MB, 39 in
-// slices of 256 KB; 32 MB 1890, 226 and 110.
+// split over host threads: one copies 20-40 GB/s, well below what NVLink-C2C
+// delivers into the staging buffers.  A slice of 256 KB is what pays for waking a
+// thread.  Copies that want every thread go to the OpenMP team (the quickest to
+// wake as a whole), smaller ones to as many helpers as they have slices for; Grace, 0.2 ms after
+// the last copy: 512 KB 8 us on one thread and 10 on two, 1 MB 21 and 14 on four,
+// 8 MB 252 and 36 on sixteen, 32 MB 1080 and 94.
 static void host_copy(void *dst, const void *src, size_t bytes) {
-    const size_t kSlice = 256u << 10;
-    const int threads = (int)std::min<size_t>((size_t)omp_get_max_threads(), bytes / kSlice);
-    if (threads < 2) {
+    const int team = omp_get_max_threads();
+    const int parts = (int)std::min<size_t>((size_t)team, bytes >> 18);
+    if (parts < 2) {
         memcpy(dst, src, bytes);
         return;
     }
-    const size_t part = ((bytes + threads - 1) / threads + 4095) & ~(size_t)4095;
-#pragma omp parallel for schedule(static) num_threads(threads)
-    for (int i = 0; i < threads; ++i) {
+    const size_t part = ((bytes + parts - 1) / parts + 4095) & ~(size_t)4095;
+    auto copy = [&](int i) {
         const size_t off = (size_t)i * part;
         if (off < bytes) memcpy((char *)dst + off, (const char *)src + off, std::min(part, bytes - off));
+    };
+    if (parts < team) {
+        HostTeam::run(parts, copy);
+        return;
     }
+#pragma omp parallel for schedule(static, 1)
+    for (int i = 0; i < parts; ++i) copy(i);
 }
 
 // Device buffer -> host, through two pinned staging buffers so that the
