@@ -769,14 +769,14 @@ static bool unitary_gates(const std::vector<const PendingGate *> &gates) {
     return true;
 }
 
-// Whether a state's stages run on the tensor cores.  complex128: from 21 lanes.
-// Forming a block's digits and a phase table costs the host more than the
-// CUDA-core program, which a circuit that is run once pays in full.  First pass and
-// repeated ones (replayed) against the CUDA-core stages, ms: 20 lanes, random 12
-// layers 4.1 and 1.15 against 3.0 and 1.87; 21 lanes, random 4 layers 1.8 and 0.88
-// against 1.6 and 1.4, QFT 1.8 and 1.2 against 2.1 and 2.0, Ising 2.5 and 1.1 against
-// 2.3 and 2.2; 22 lanes 2.0 and 1.1 against 2.3 and 2.1, 2.1 and 1.6 against 3.1 and
-// 3.0, 2.8 and 1.2 against 3.3 and 3.2.
+// Whether a state's stages run on the tensor cores.  complex128: from the size on
+// at which a circuit's first pass gains, too.  Forming a block's digits and a phase
+// table costs the host more than the CUDA-core program, which a circuit that is run once
+// pays in full.  First passes (and repeated ones, replayed) with digits / on the
+// CUDA cores, ms: 20 lanes, random 4 layers 1.29 (0.61) / 1.13 (0.81), 20 layers 6.28
+// (1.96) / 4.95 (2.92), QFT 1.32 (0.83) / 1.22 (1.13), Ising 1.65 (0.85) / 1.39 (1.29);
+// 21 lanes, 1.66 (0.90) / 1.70 (1.40), 6.30 (2.66) / 7.01 (5.02), 1.69 (1.22) / 2.10 (1.98), 2.01
+// (1.19) / 2.31 (2.21); 23 lanes, 2.74 / 4.47, 9.1 / 18.3, 3.07 / 6.05, 3.35 / 6.34.
 constexpr int kDigitLanes = 21;
 static bool tensor_stages_pay(const Device &d, const States *s) {
     return d.tensor_blocks &&

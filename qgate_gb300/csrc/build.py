@@ -23,6 +23,8 @@ ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 CU_SOURCES = ['gates.cu', 'reduce.cu', 'fused.cu', 'adjoint.cu', 'batch.cu', 'noalloc.cu', 'tcstage.cu',
               'dstage.cu']
 CXX_SOURCES = ['api.cpp', 'adjoint_host.cpp', 'tcplan.cpp']
+# operands are formed while the GPU waits: vectorised, a third of the time of -O2
+CXX_OPT = {'tcplan.cpp': '-O3'}
 
 
 def _cuda_home():
@@ -82,7 +84,7 @@ def build(force=False, verbose=False, ptxas_verbose=False):
         objs.append(o)
         if force or _stale(o, s):
             cxx = os.environ.get('CXX', 'g++')
-            jobs.append([cxx, '-O2', '-std=c++17', '-fPIC', '-Wall', '-fopenmp', '-c', s, '-o', o] + inc)
+            jobs.append([cxx, CXX_OPT.get(src, '-O2'), '-std=c++17', '-fPIC', '-Wall', '-fopenmp', '-c', s, '-o', o] + inc)
     outputs = []
     if jobs:
         with concurrent.futures.ThreadPoolExecutor(max_workers=len(jobs)) as ex:

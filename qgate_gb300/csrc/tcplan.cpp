@@ -8,6 +8,8 @@
 #include <cstring>
 #include <cmath>
 
+#include "host_team.h"
+
 namespace qg {
 
 unsigned long long gate_qmask(const PendingGate &g) {
@@ -305,10 +307,8 @@ static void tc_operand(const std::complex<double> *U, unsigned short *bh, unsign
 // returned: 0 for a unitary), each entry cut into kDigits balanced radix-2^10
 // digits, b1 = rint(x 2^10) and every next one rint of 2^10 times the rest
 // (exact in FP64; the last to quarters), in the chunks described at
-// kDigitOpBytes.  low: whether the 1-norm of some column of b2 or b3 passes
-// 3/4 of its largest, 64 * 512 (the stage's sums then need smaller inputs).
-static int tc_operand_digits(const std::complex<double> *U, unsigned short *out, bool *low) {
-    *low = false;
+// kDigitOpBytes.
+static int tc_digit_exponent(const std::complex<double> *U) {
     double norm2 = 0.;
     for (int o = 0; o < 32; ++o) {
         double row = 0.;
@@ -320,6 +320,12 @@ static int tc_operand_digits(const std::complex<double> *U, unsigned short *out,
     if (norm2 > 0.) {
         std::frexp(std::sqrt(norm2) * (1. - 1e-9), &e);
     }
+    return e;
+}
+// The digits.  Returns whether the 1-norm of some column of b2 or b3 passes 3/4 of
+// its largest, 64 * 512 (the stage's sums then need smaller inputs).
+static bool tc_digit_rows(const std::complex<double> *U, int e, unsigned short *out) {
+    bool low = false;
     const double scale = std::ldexp(1., 10 - e);
     // b in FP16: |b| <= 1024, exact (the table's index is 4 b + 4096).  The
     // last digit keeps quarters, which FP16 holds up to 512: two more bits.
@@ -329,35 +335,36 @@ static int tc_operand_digits(const std::complex<double> *U, unsigned short *out,
         return t;
     }();
     for (int o = 0; o < 32; ++o) {
-        int sum[kDigits] = {0};  // four times the columns' 1-norms
-        for (int i = 0; i < 32; ++i)
-            for (int part = 0; part < 2; ++part) {
-                // (row, column) of D = A B are (k, n): re at (2i, 2o) and
-                // (2i + 1, 2o + 1), im at (2i, 2o + 1), -im at (2i + 1, 2o)
-                double x = (part ? U[o * 32 + i].imag() : U[o * 32 + i].real()) * scale;
-                const size_t at = (size_t)(4 * (o >> 4) + (i >> 3)) * (kDigitChunkBytes / 2) +
-                                  (i % 8 / 4) * 1280 + (2 * o & 31) / 8 * 64 + (2 * o & 7) * 8 +
-                                  2 * (i & 3);
-                unsigned short *p = out + at;
-                for (int j = 0; j < kDigits; ++j, p += 256) {
-                    // rint(x) for |x| <= 1024 by the 1.5 * 2^52 addition
-                    // (to quarters: 1.5 * 2^50)
-                    const double c = j + 1 < kDigits ? 6755399441055744. : 1688849860263936.;
-                    const double b = (x + c) - c;
-                    x = (x - b) * 1024.;
-                    const int v = (int)(4. * b);
-                    sum[j] += v < 0 ? -v : v;
-                    if (part == 0) {
-                        p[0] = p[9] = f16[4096 + v];
-                    } else {
-                        p[8] = f16[4096 + v];
-                        p[1] = f16[4096 - v];
-                    }
-                }
+        double x[64];  // the row's parts, re and im
+        for (int k = 0; k < 32; ++k) {
+            x[2 * k] = U[o * 32 + k].real() * scale;
+            x[2 * k + 1] = U[o * 32 + k].imag() * scale;
+        }
+        for (int j = 0; j < kDigits; ++j) {
+            // rint(x) for |x| <= 1024 by the 1.5 * 2^52 addition
+            // (to quarters: 1.5 * 2^50)
+            const double c = j + 1 < kDigits ? 6755399441055744. : 1688849860263936.;
+            int v[64], sum = 0;  // four times the digits, and the column's 1-norm
+            for (int k = 0; k < 64; ++k) {
+                const double b = (x[k] + c) - c;
+                x[k] = (x[k] - b) * 1024.;
+                v[k] = (int)(4. * b);
             }
-        *low = *low || std::max(sum[1], sum[2]) > 4 * 24576;
+            for (int k = 0; k < 64; ++k) sum += v[k] < 0 ? -v[k] : v[k];
+            if (j == 1 || j == 2) low = low || sum > 4 * 24576;
+            // (row, column) of D = A B are (k, n): re at (2i, 2o) and
+            // (2i + 1, 2o + 1), im at (2i, 2o + 1), -im at (2i + 1, 2o)
+            for (int i = 0; i < 32; ++i) {
+                unsigned short *p = out + (size_t)(4 * (o >> 4) + (i >> 3)) * (kDigitChunkBytes / 2) +
+                                    (i % 8 / 4) * 1280 + j * 256 + (2 * o & 31) / 8 * 64 +
+                                    (2 * o & 7) * 8 + 2 * (i & 3);
+                p[0] = p[9] = f16[4096 + v[2 * i]];
+                p[8] = f16[4096 + v[2 * i + 1]];
+                p[1] = f16[4096 - v[2 * i + 1]];
+            }
+        }
     }
-    return e;
+    return low;
 }
 
 // Bias compensation for the tensor core's accumulator.  The FP32 accumulator
@@ -522,29 +529,61 @@ static TcLayout tc_choose_layout(unsigned lanes, unsigned next_lanes, const TcLa
     return c;
 }
 
-// U (32x32, row-major) of a block's gates in the amplitude order of `lay`.
+// U (32x32, row-major) of a block's gates in the amplitude order of `lay`.  Real
+// arithmetic on the two parts' planes, which is vectorised (a complex product's
+// checks for NaN are not); X exchanges rows and a diagonal gate scales them.
 static void tc_block_matrix(const std::vector<const PendingGate *> &gates, const TileLanes &tl,
                             const TcLayout &lay, std::complex<double> *U) {
-    typedef std::complex<double> cd;
     int bit_of[64];
     for (int p = 0; p < 64; ++p) bit_of[p] = -1;
     for (int k = 0; k < 5; ++k) bit_of[lay.amps[k]] = k;
-    for (int i = 0; i < 1024; ++i) U[i] = (i / 32 == i % 32) ? cd(1, 0) : cd(0, 0);
+    struct Row {
+        double re[32], im[32];
+    };
+    Row u[32];
+    for (int r = 0; r < 32; ++r)
+        for (int c = 0; c < 32; ++c) {
+            u[r].re[c] = r == c ? 1. : 0.;
+            u[r].im[c] = 0.;
+        }
+    static const double x[8] = {0., 0., 1., 0., 1., 0., 0., 0.};
+    auto scale = [](Row &row, double re, double im) {
+        if (re == 1. && im == 0.) return;
+        for (int c = 0; c < 32; ++c) {
+            const double a = row.re[c], b = row.im[c];
+            row.re[c] = re * a - im * b;
+            row.im[c] = re * b + im * a;
+        }
+    };
     for (auto *g : gates) {
         const int tb = 1 << bit_of[tl.local_of[g->target]];
         int cm = 0;
         for (int c : g->controls) cm |= 1 << bit_of[tl.local_of[c]];
-        const cd m00(g->m.v[0], g->m.v[1]), m01(g->m.v[2], g->m.v[3]), m10(g->m.v[4], g->m.v[5]),
-            m11(g->m.v[6], g->m.v[7]);
+        const double *v = g->m.v;
+        const double m0 = v[0], m1 = v[1], m2 = v[2], m3 = v[3], m4 = v[4], m5 = v[5], m6 = v[6],
+                     m7 = v[7];
+        const bool swap = memcmp(v, x, sizeof(x)) == 0;
         for (int r = 0; r < 32; ++r) {
             if ((r & tb) || (r & cm) != cm) continue;
-            for (int c = 0; c < 32; ++c) {
-                cd a0 = U[r * 32 + c], a1 = U[(r | tb) * 32 + c];
-                U[r * 32 + c] = m00 * a0 + m01 * a1;
-                U[(r | tb) * 32 + c] = m10 * a0 + m11 * a1;
+            Row &p = u[r], &q = u[r | tb];
+            if (swap) {
+                std::swap(p, q);
+            } else if (g->diag) {
+                scale(p, m0, m1);
+                scale(q, m6, m7);
+            } else {
+                for (int c = 0; c < 32; ++c) {
+                    const double a = p.re[c], b = p.im[c], e = q.re[c], f = q.im[c];
+                    p.re[c] = (m0 * a - m1 * b) + (m2 * e - m3 * f);
+                    p.im[c] = (m0 * b + m1 * a) + (m2 * f + m3 * e);
+                    q.re[c] = (m4 * a - m5 * b) + (m6 * e - m7 * f);
+                    q.im[c] = (m4 * b + m5 * a) + (m6 * f + m7 * e);
+                }
             }
         }
     }
+    for (int r = 0; r < 32; ++r)
+        for (int c = 0; c < 32; ++c) U[r * 32 + c] = {u[r].re[c], u[r].im[c]};
 }
 
 // Fills a block of fewer than 5 lanes: lanes of the source layout's warp
@@ -700,19 +739,23 @@ void tc_phase_values(const TcOp &op, const TileLanes &tl, const std::vector<int>
     for (int k = 0; k < u; ++k) bit_of[positions[k]] = k;
     // gate by gate over the entries it changes (a QFT's controlled phases: a quarter;
     // entry by entry over all gates, a 21-lane complex128 QFT's first pass took 3.2 ms
-    // instead of 1.8)
+    // instead of 1.8); real arithmetic as in tc_block_matrix
     const unsigned all = (1u << u) - 1u;
     std::fill(table, table + (1u << u), cd(1., 0.));
+    double *const t = (double *)table;
     for (auto *g : op.gates) {
         unsigned on = 0;
         for (int c : g->controls) on |= 1u << bit_of[tl.local_of[c]];
         const unsigned target = 1u << bit_of[tl.local_of[g->target]];
         for (int side = 0; side < 2; ++side) {
-            const cd f(g->m.v[6 * side], g->m.v[6 * side + 1]);
-            if (f == cd(1., 0.)) continue;
+            const double re = g->m.v[6 * side], im = g->m.v[6 * side + 1];
+            if (re == 1. && im == 0.) continue;
             const unsigned fixed = on | (side ? target : 0u), free = all & ~(on | target);
             for (unsigned k = free;; k = (k - 1u) & free) {
-                table[fixed | k] *= f;
+                double *e = t + 2 * (size_t)(fixed | k);
+                const double a = e[0], b = e[1];
+                e[0] = a * re - b * im;
+                e[1] = a * im + b * re;
                 if (k == 0) break;
             }
         }
@@ -905,6 +948,11 @@ static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops,
     for (int k = 0; k < 5; ++k) desc.in_e[k] = desc.dep_hi[1 << k];
     desc.sets[nb + 1] = tc_slots(cur, t, [&](unsigned ti) { return host_swz(ti, prec); });
     std::complex<double> U[1024];
+    struct Dense {  // complex128 blocks: their operands are formed at the end
+        int b;
+        TcLayout lay;
+    };
+    std::vector<Dense> dense;
     for (int b = 0; b < nb; ++b) {
         const TcOp &op = ops[b0 + b];
         if (op.cross) {
@@ -990,17 +1038,27 @@ static void tc_plan_launch_ordered(const TileLanes &tl, int n, const TcOps &ops,
         desc.sets[b] = tc_slots(cur, t, [&](unsigned ti) { return tc_operand_slot(lay, ti); });
         if (order)
             for (int k = 0; k < 5; ++k) order->amps[b][k] = (signed char)lay.amps[k];
-        tc_block_matrix(op.gates, tl, lay, U);
-        unsigned short *o = (unsigned short *)(buf + desc.op_off[b]);
         if (prec == kFP64) {
-            bool low;
-            desc.op_exp[b] = (short)tc_operand_digits(U, o, &low);
-            desc.op_low[b] = low ? 1 : 0;
+            dense.push_back({b, lay});
         } else {
+            tc_block_matrix(op.gates, tl, lay, U);
+            unsigned short *o = (unsigned short *)(buf + desc.op_off[b]);
             tc_compensate(U);
             tc_operand(U, o, o + 64 * 64);
         }
         cur = lay;
+    }
+    if (!dense.empty()) {
+        // The digits of complex128 blocks, which a circuit that runs once waits
+        // for: 20 us a block on Grace
+        HostTeam::run((int)dense.size(), [&](int i) {
+            std::complex<double> u[1024];
+            const int b = dense[i].b;
+            tc_block_matrix(ops[b0 + b].gates, tl, dense[i].lay, u);
+            const int e = tc_digit_exponent(u);
+            desc.op_exp[b] = (short)e;
+            desc.op_low[b] = tc_digit_rows(u, e, (unsigned short *)(buf + desc.op_off[b])) ? 1 : 0;
+        });
     }
     desc.sets[nb] = tc_slots(cur, t, [&](unsigned ti) { return host_swz(ti, prec); });
     desc.direct_out = direct_out ? 1 : 0;

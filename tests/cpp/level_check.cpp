@@ -54,8 +54,7 @@ int main() {
             for (int i = 0; i < 32; ++i)
                 U[o * 32 + i] = std::polar(1. / std::sqrt(32.), phi) *
                                 (double)(__builtin_popcount(o & i) & 1 ? -1 : 1);
-        bool low;
-        tc_operand_digits(U, B.data(), &low);
+        const bool low = tc_digit_rows(U, tc_digit_exponent(U), B.data());
         lows += low;
         for (int o = 0; o < 64; ++o) {
             double n1[3] = {0, 0, 0}, n2 = 0;  // 1-norms of B1..B3, 2-norm of B1
