@@ -1187,9 +1187,13 @@ static bool marginal_one_state(int prec, double *out, int n_lanes, int n_hidden,
     }
     MargDesc d;
     d.nvis = d.nhid = 0;
+    int low_hidden = 0;
+    bool in_order = true;  // the visible lanes are the lowest ones, in order
     for (int l = 0; l < n; ++l) {
         const int e = g.ext[l];
+        if (e < n_lanes && e != l) in_order = false;
         if (l < 8) {
+            low_hidden += e >= n_lanes;
             d.low_ext[l] = (signed char)(e < n_lanes ? e : -1);
         } else if (e < n_lanes) {
             d.vis_pos[d.nvis] = (signed char)l;
@@ -1199,6 +1203,14 @@ static bool marginal_one_state(int prec, double *out, int n_lanes, int n_hidden,
         }
     }
     if (d.nvis > 24) return false;
+    // CTAs with one run or two of 256 amplitudes do little beside starting and adding
+    // threads up, which counts once they outnumber what the GPU holds: from 21 lanes on
+    // k_marginal takes those that it runs faster.  c64 / c128, ms, k_marginal and this:
+    // 28 lanes, five low lanes hidden 2.60 and 3.82 / 2.95 and 3.89, seven and one high
+    // 2.56 and 2.91 / 2.91 and 2.84, the highest two (in order) 1.01 and 1.15 / 1.49
+    // and 1.27; 18 lanes, the same: 0.016 and 0.011, 0.037 and 0.010, 0.011 and 0.009.
+    if (n >= 21 && (d.nhid == 0 || (d.nhid == 1 && low_hidden >= 6) || (in_order && d.nhid <= 2)))
+        return false;
     // enough CTAs to fill the GPU evenly (8192, seven waves), each with at least
     // eight runs, and no more partial sums than the scratch holds
     int gl = 0;
