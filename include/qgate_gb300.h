@@ -224,8 +224,13 @@ int qg_set_pageable_copy(int on);
 int qg_set_pool_guide_index_shift(int k);
 /* Extension: status word of the tensor-core stage kernels after a
  * synchronize: 0 = every bounded wait completed; nonzero = a wait gave up
- * (that stage's tiles were left unchanged).  reset != 0 clears it. */
+ * (that stage's tiles were left unchanged; bits 8 and up: the complex128
+ * stage).  Until reset != 0 clears it, later stages leave states as they are
+ * and every call that returns results fails with QG_ERR_TIMEOUT. */
 int qg_tensor_stage_status(int reset, int *status);
+/* Extension: sets that status as a stage kernel would whose wait gave up (for
+ * tests of what follows). */
+int qg_tensor_stage_raise(int status);
 /* Extension: counters of the gate path since the last reset
  * {gates, passes, bytes_moved}. */
 int qg_gate_stats(int64_t *gates, int64_t *passes, int64_t *bytes, int reset);

@@ -67,6 +67,7 @@ SIGNATURES = {
     'qg_trace_stats': [_i64p, _i64p, _i],
     'qg_set_tensor_blocks': [_i],
     'qg_tensor_stage_status': [_i, _ip],
+    'qg_tensor_stage_raise': [_i],
     'qg_set_host_direct': [_i],
     'qg_set_pageable_copy': [_i],
     'qg_set_pool_guide_index_shift': [_i],
@@ -198,6 +199,8 @@ def grouping_stats(reset=False):
 
 
 def tensor_stage_status(reset=False):
+    """Nonzero once a tensor stage's bounded wait has given up; calls that return
+    results raise then, until this is called with reset=True."""
     v = ctypes.c_int(0)
     check(lib.qg_tensor_stage_status(1 if reset else 0, ctypes.byref(v)))
     return v.value

@@ -667,6 +667,7 @@ static void adjoint_run(int prec, int n, std::vector<Op> &ops, const double *par
             QG_CUDA(cudaMemcpyAsync(sums.data(), dsums, sizeof(double) * sums.size(),
                                     cudaMemcpyDeviceToHost, st));
         QG_CUDA(cudaStreamSynchronize(st));
+        engine_check_stages();
         if (G_out) {
             std::fill(G_out, G_out + (size_t)batch * n_params, 0.);
             for (int b = 0; b < batch; ++b)

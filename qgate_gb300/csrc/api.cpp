@@ -253,6 +253,9 @@ struct Device {
     // needed.
     static constexpr int kMarkLanes = 34;
     TileMarks marks = {nullptr, nullptr};
+    // What the tensor stages' waits that gave up have reported (host memory that the
+    // device writes); every call that returns results looks at it.
+    volatile unsigned *stage_status = nullptr;
     // Pinned staging of a batch's programs (grown on demand; reused by the
     // next batch, which starts after this one's results are read).
     unsigned char *h_batch = nullptr;
@@ -308,6 +311,13 @@ static void device_init(int device_id, long long limit) {
     QG_CUDA(cudaMallocHost(&d.h_result, sizeof(double) * 16));
     QG_CUDA(cudaMalloc(&d.marks.count, 2 * sizeof(unsigned)));
     QG_CUDA(cudaMemset(d.marks.count, 0, 2 * sizeof(unsigned)));
+    void *status = nullptr, *status_dev = nullptr;
+    QG_CUDA(cudaHostAlloc(&status, sizeof(unsigned), cudaHostAllocMapped));
+    QG_CUDA(cudaHostGetDevicePointer(&status_dev, status, 0));
+    d.stage_status = (volatile unsigned *)status;
+    *d.stage_status = 0u;
+    tstage_status_host((unsigned *)status_dev);
+    dstage_status_host((unsigned *)status_dev);
     for (int i = 0; i < 2; ++i) {
         QG_CUDA(cudaMallocHost(&d.h_stage[i], Device::kStageBytes));
         QG_CUDA(cudaEventCreateWithFlags(&d.ev[i], cudaEventDisableTiming));
@@ -331,6 +341,8 @@ static Device &dev() {
 }
 
 cudaStream_t engine_stream() { return dev().stream; }
+static void check_stages(const Device &d);
+void engine_check_stages() { check_stages(dev()); }
 void *engine_alloc(size_t bytes) { return dev().arena.alloc(bytes); }
 bool tensor_stages_enabled() { return dev().tensor_blocks; }
 void engine_free(void *p) { g_dev.arena.release(p); }
@@ -1220,9 +1232,19 @@ static void flush_all() {
     for (States *s : g_dev.states) flush(s);
 }
 
+// Before results go to the caller (the stream's work is done): once a tensor
+// stage's wait has given up, amplitudes are not what the gates make of them.
+static void check_stages(const Device &d) {
+    const unsigned s = *d.stage_status;
+    if (s)
+        fail(QG_ERR_TIMEOUT, "a tensor stage's wait gave up (status 0x%x): states it worked on are "
+             "not valid; qg_tensor_stage_status(1, ..) clears this.", s);
+}
+
 static double read_result(Device &d, double *d_val) {
     QG_CUDA(cudaMemcpyAsync(d.h_result, d_val, sizeof(double), cudaMemcpyDeviceToHost, d.stream));
     QG_CUDA(cudaStreamSynchronize(d.stream));
+    check_stages(d);
     return d.h_result[0];
 }
 
@@ -1281,6 +1303,7 @@ static void staged_d2h(Device &d, void *host, idx_t count, size_t item, F produc
     if (kernel_output && d.host_direct) {
         produce(0, count, host);
         QG_CUDA(cudaStreamSynchronize(d.stream));
+        check_stages(d);
         return;
     }
     const size_t bytes = (size_t)count * item;
@@ -1303,6 +1326,7 @@ static void staged_d2h(Device &d, void *host, idx_t count, size_t item, F produc
             throw;
         }
         d.arena.release(dbuf);
+        check_stages(d);
         return;
     }
     idx_t chunk = (idx_t)(Device::kStageBytes / item);
@@ -1336,6 +1360,7 @@ static void staged_d2h(Device &d, void *host, idx_t count, size_t item, F produc
     }
     d.arena.release(dbuf[0]);
     d.arena.release(dbuf[1]);
+    check_stages(d);
 }
 
 // ------------------------------------------------------------ gather descriptors
@@ -1737,6 +1762,7 @@ int qg_qubit_processor_synchronize(qg_handle h) {
     Device &d = dev();
     flush_all();
     QG_CUDA(cudaStreamSynchronize(d.stream));
+    check_stages(d);
     QG_END
 }
 
@@ -2198,12 +2224,22 @@ int qg_set_tensor_blocks(int on) {
     QG_END
 }
 
+int qg_tensor_stage_raise(int status) {
+    QG_BEGIN
+    Device &d = dev();
+    if (status < 0 || status > 0xffff) fail(QG_ERR_VALUE, "bad stage status %d.", status);
+    if (status & 0xff) tstage_raise((unsigned)status & 0xffu, d.stream);
+    if (status >> 8) dstage_raise((unsigned)status >> 8, d.stream);
+    QG_END
+}
+
 int qg_tensor_stage_status(int reset, int *status) {
     QG_BEGIN
     Device &d = dev();
     flush_all();
     QG_CUDA(cudaStreamSynchronize(d.stream));
     *status = tstage_status(reset != 0) | (dstage_status(reset != 0) << 8);
+    if (reset) *d.stage_status = 0u;
     QG_END
 }
 
@@ -3006,6 +3042,7 @@ int qg_qubits_states_getter_create_sampling_pool(qg_handle hg, const int *lane_t
             QG_CUDA(cudaMemcpyAsync(d.h_result + 1, guide.long_count, sizeof(unsigned),
                                     cudaMemcpyDeviceToHost, d.stream));
         QG_CUDA(cudaStreamSynchronize(d.stream));
+        check_stages(d);
         memcpy(&total, d.h_result, 8);
         if (guide.g) {
             unsigned long_count = 0;

@@ -87,7 +87,7 @@
 
 namespace qg {
 
-__device__ unsigned g_ds_status;
+__device__ StageStatus g_ds_status;
 
 namespace {
 
@@ -336,10 +336,10 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
     const int nb = d.nblocks;
 
     if ((smem_u32(smraw) & 1023u) != 0u) {
-        if (tid == 0) atomicOr(&g_ds_status, 4u);
+        if (tid == 0) report_stage(&g_ds_status, 4u, 4u << 8);
         return;
     }
-    if (tid == 0) stop_sh = *(volatile unsigned *)&g_ds_status != 0u;
+    if (tid == 0) stop_sh = *(volatile unsigned *)&g_ds_status.bits != 0u;
     __syncthreads();
     if (stop_sh) return;
     __syncthreads();
@@ -536,7 +536,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
                 }
             }
             if (!ok && lane) {
-                atomicOr(&g_ds_status, 1u);
+                report_stage(&g_ds_status, 1u, 1u << 8);
                 mma_commit(smem_u32(&bar_end));
                 mbar_wait(smem_u32(&bar_end), 0u);
             }
@@ -755,7 +755,7 @@ k_dstage(uint4 *__restrict__ s, const __grid_constant__ TcStageDesc d, int tiles
             }
             if (!ok) {
                 abort_sh[g] = 1;
-                atomicOr(&g_ds_status, 2u);
+                report_stage(&g_ds_status, 2u, 2u << 8);
             }
             {
                 // the smallest amplitude (high words; the bits of either part stand
@@ -925,11 +925,23 @@ void launch_dstage(void *state, const TcStageDesc &d, const TileMarks &marks, cu
     QG_CUDA(cudaGetLastError());
 }
 
+__global__ void k_raise_dstage(unsigned bits) { report_stage(&g_ds_status, bits, bits << 8); }
+
+void dstage_status_host(unsigned *word) {
+    const StageStatus s = {0u, word};
+    QG_CUDA(cudaMemcpyToSymbol(g_ds_status, &s, sizeof(s)));
+}
+
+void dstage_raise(unsigned bits, cudaStream_t stream) {
+    k_raise_dstage<<<1, 1, 0, stream>>>(bits);
+    QG_CUDA(cudaGetLastError());
+}
+
 int dstage_status(bool reset) {
     unsigned v = 0;
     QG_CUDA(cudaMemcpyFromSymbol(&v, g_ds_status, sizeof(v)));
     if (reset && v) {
-        unsigned z = 0;
+        const unsigned z = 0;
         QG_CUDA(cudaMemcpyToSymbol(g_ds_status, &z, sizeof(z)));
     }
     return (int)v;

@@ -223,8 +223,14 @@ int dstage_status(bool reset);
 constexpr int kMaxPhaseLanes = 12;
 void launch_phase_f64(void *state, int n, const int *lanes, int n_lanes, const void *table,
                       cudaStream_t stream);
-// Status word of the tensor stage kernels (nonzero: a bounded wait gave up).
+// Status words of the tensor stage kernels (nonzero: a bounded wait gave up).  Each
+// kernel also sets its bits in the host word given to *_status_host (k_dstage: from bit
+// 8 on); *_raise sets them as a kernel would.
 int tstage_status(bool reset);
+void tstage_status_host(unsigned *word);
+void tstage_raise(unsigned bits, cudaStream_t stream);
+void dstage_status_host(unsigned *word);
+void dstage_raise(unsigned bits, cudaStream_t stream);
 
 // XOR swizzle of shared-memory element slots (see qg_regstage.cuh):
 // 16 slots per 128-byte row for complex64, 8 for complex128.  An involution.
@@ -401,6 +407,7 @@ int batch_persistent_ctas();
 cudaStream_t engine_stream();
 void *engine_alloc(size_t bytes);
 void engine_free(void *p);
+void engine_check_stages();  // throws once a tensor stage's wait has given up
 // Pinned host memory of at least `bytes`, kept for the next caller; its contents
 // last until the caller's call returns.
 void *engine_pinned(size_t bytes);

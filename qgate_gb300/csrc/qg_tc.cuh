@@ -32,6 +32,19 @@ __device__ __forceinline__ void mma_f16(unsigned dtmem, uint64_t a, uint64_t b, 
         : "memory");
 }
 
+// A wait of a tensor stage gave up: its status word, which later launches look at,
+// and the host's, which calls that return results look at (its device address, set
+// when the engine starts).
+struct StageStatus {
+    unsigned bits;
+    unsigned *host;
+};
+__device__ __forceinline__ void report_stage(StageStatus *s, unsigned bits, unsigned host_bits) {
+    atomicOr(&s->bits, bits);
+    unsigned *h = *(unsigned *volatile *)&s->host;
+    if (h) atomicOr_system(h, host_bits);
+}
+
 // One lane of a converged warp (the same one at every call): code that the
 // whole warp walks keeps descriptors in uniform registers, where tcgen05.mma
 // takes them; issued from a single thread's branch the same products cost 100

@@ -49,7 +49,7 @@
 
 namespace qg {
 
-__device__ unsigned g_tc_status;
+__device__ StageStatus g_tc_status;
 
 namespace {
 
@@ -162,10 +162,10 @@ k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, 
 
     // The operand atoms must be 1024-byte aligned for the 128-byte swizzle.
     if ((smem_u32(smraw) & 1023u) != 0u) {
-        if (tid == 0) atomicOr(&g_tc_status, 4u);
+        if (tid == 0) report_stage(&g_tc_status, 4u, 4u);
         return;
     }
-    if (tid == 0) abort_sh[0] = *(volatile unsigned *)&g_tc_status != 0u;
+    if (tid == 0) abort_sh[0] = *(volatile unsigned *)&g_tc_status.bits != 0u;
     __syncthreads();
     if (abort_sh[0]) return;
     __syncthreads();
@@ -245,7 +245,7 @@ k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, 
                 // register table lives in the warps' lanes.
                 if (!t_ready) {
                     t_ready = mbar_wait(bb, 0u);
-                    if (!t_ready) atomicOr(&g_tc_status, 1u);
+                    if (!t_ready) report_stage(&g_tc_status, 1u, 1u);
                 }
                 const TcCrossHdr &xh = *(const TcCrossHdr *)(Bs + d.op_off[b]);
                 const TcCrossRec *xr = (const TcCrossRec *)(Bs + d.op_off[b] + sizeof(TcCrossHdr));
@@ -321,7 +321,7 @@ k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, 
                 // itself (bounded; a wait that gives up is reported).
                 if (!t_ready) {
                     t_ready = mbar_wait(bb, 0u);
-                    if (!t_ready) atomicOr(&g_tc_status, 1u);
+                    if (!t_ready) report_stage(&g_tc_status, 1u, 1u);
                 }
                 const float2 *tab = (const float2 *)(Bs + d.op_off[b]);
 #pragma unroll
@@ -385,7 +385,7 @@ k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, 
                     }
                     mma_commit(bmma);
                 } else {
-                    atomicOr(&g_tc_status, 1u);
+                    report_stage(&g_tc_status, 1u, 1u);
                     abort_sh[g] = 1;
                     mbar_arrive(bmma);
                 }
@@ -394,7 +394,7 @@ k_tstage(const float2 *src, float2 *dst, const __grid_constant__ TcStageDesc d, 
             phase ^= 1u;
             if (!got) {
                 abort_sh[g] = 1;
-                atomicOr(&g_tc_status, 2u);
+                report_stage(&g_tc_status, 2u, 2u);
             }
             // One decision for the whole group, so that its threads leave
             // together.
@@ -564,11 +564,23 @@ void launch_tstage(void *state, const TcStageDesc &d, cudaStream_t stream, bool 
     QG_CUDA(cudaGetLastError());
 }
 
+__global__ void k_raise_tstage(unsigned bits) { report_stage(&g_tc_status, bits, bits); }
+
+void tstage_status_host(unsigned *word) {
+    const StageStatus s = {0u, word};
+    QG_CUDA(cudaMemcpyToSymbol(g_tc_status, &s, sizeof(s)));
+}
+
+void tstage_raise(unsigned bits, cudaStream_t stream) {
+    k_raise_tstage<<<1, 1, 0, stream>>>(bits);
+    QG_CUDA(cudaGetLastError());
+}
+
 int tstage_status(bool reset) {
     unsigned v = 0;
     QG_CUDA(cudaMemcpyFromSymbol(&v, g_tc_status, sizeof(v)));
     if (reset && v) {
-        unsigned z = 0;
+        const unsigned z = 0;
         QG_CUDA(cudaMemcpyToSymbol(g_tc_status, &z, sizeof(z)));
     }
     return (int)v;
