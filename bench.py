@@ -707,7 +707,7 @@ def run_c4(args, rt, nat):
         autotune.apply(cached)
     else:
         nat.set_fusion(12)
-        nat.set_tensor_blocks(True)
+        nat.set_tensor_blocks(None)
     n1 = args.c4_random_qubits
     if n1 > 0:  # 0 skips it
         ops1 = circuit(n1, 30, seed_angles=40, seed_perm=40)

@@ -193,11 +193,11 @@ int qg_set_fusion_params(int prec, int tile_lanes, int reg_lanes, int cost_budge
  * per row), which keeps more warps resident per SM for the CUDA-core stage
  * and fewer, busier threads for the tensor-core stage. */
 int qg_set_stage_pipelining(int on);
-/* Extension: 1 runs complex64 stages of 12- or 13-lane tiles and complex128
- * stages of 12-lane tiles as fused 5-lane blocks (32x32 complex matrices) on
- * the tensor cores, 0 on the register-resident CUDA-core stage kernel.  The
- * default (before the first call, and after qg_set_fusion(0)) is 1 for
- * complex64, and for complex128 states of 21 lanes and more.  No reference counterpart: the
+/* Extension: 1 (the default, also after qg_set_fusion(0)) runs complex64 stages
+ * of 12- or 13-lane tiles, and complex128 stages of 12-lane tiles of states of 21
+ * lanes and more, as fused 5-lane blocks (32x32 complex matrices) on the tensor
+ * cores; 2 complex128 states of every size too; 0 runs all on the
+ * register-resident CUDA-core stage kernel.  No reference counterpart: the
  * reference applies one gate per pass
  * (qgate/simulator/src/CUDAQubitProcessor.cpp:271, applyGate). */
 int qg_set_tensor_blocks(int on);

@@ -170,8 +170,9 @@ def set_fusion_params(prec, tile_lanes, reg_lanes, cost_budget=0):
 def set_tensor_blocks(on):
     """Run stages of 12-lane tiles (complex64 13 too) as fused 5-lane blocks on
     the tensor cores (tcgen05 kind::f16 on split FP16 operands; complex128 on
-    digits).  By default: complex64, and complex128 from 21 lanes."""
-    call('qg_set_tensor_blocks', 1 if on else 0)
+    digits): None (the default) complex64, and complex128 from 21 lanes; True
+    states of every size in both precisions; False none."""
+    call('qg_set_tensor_blocks', 1 if on is None else 2 if on else 0)
 
 
 def set_trace_replay(on):

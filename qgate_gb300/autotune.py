@@ -81,10 +81,16 @@ def _prec(dtype):
     return nat.PREC_FP64 if dtype == np.float64 else nat.PREC_FP32
 
 
+def _set_tensor(prec, tensor):
+    """Tensor stages on or off for a precision's candidate: complex64 ones leave
+    complex128 states at their default."""
+    nat.set_tensor_blocks(bool(tensor) if prec == nat.PREC_FP64 or not tensor else None)
+
+
 def apply(best):
     nat.set_fusion_params(best['prec'], best['tile_lanes'], best['reg_lanes'],
                           best['cost_budget'])
-    nat.set_tensor_blocks(best.get('tensor', 0))
+    _set_tensor(best['prec'], best.get('tensor', 0))
     nat.call('qg_set_stage_pipelining', int(best.get('prefetch', 0)))
 
 
@@ -113,7 +119,7 @@ def _time_candidates(n_lanes, dtype, ops, repeats, cands):
         if tile > n_lanes:
             continue
         nat.set_fusion_params(prec, tile, rl, budget)
-        nat.set_tensor_blocks(tensor)
+        _set_tensor(prec, tensor)
         nat.call('qg_set_stage_pipelining', prefetch)
         run()
         t0 = time.perf_counter()

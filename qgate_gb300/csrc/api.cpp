@@ -2217,10 +2217,11 @@ int qg_set_fusion_params(int prec, int tile_lanes, int reg_lanes, int cost_budge
 
 int qg_set_tensor_blocks(int on) {
     QG_BEGIN
+    if (on < 0 || on > 2) on = 1;  // (any other value was "on" always)
     flush_all();
     g_dev.settings_version += 1;  // compiled circuits re-plan
     g_dev.tensor_blocks = on != 0;
-    g_dev.digits_always = on != 0;
+    g_dev.digits_always = on == 2;
     QG_END
 }
 

@@ -18,3 +18,13 @@ def rt():
     library is missing, so a missing build cannot pass silently."""
     from qgate_gb300 import gb300runtime
     return gb300runtime
+
+
+@pytest.fixture(autouse=True)
+def _default_settings(request):
+    """GPU tests leave the fusion settings as they were, so that what the next one
+    runs on does not depend on their order."""
+    yield
+    if request.node.get_closest_marker('gpu'):
+        from qgate_gb300 import _native
+        _native.set_fusion(0)
