@@ -785,10 +785,10 @@ static bool unitary_gates(const std::vector<const PendingGate *> &gates) {
 // at which a circuit's first pass gains, too.  Forming a block's digits and a phase
 // table costs the host more than the CUDA-core program, which a circuit that is run once
 // pays in full.  First passes (and repeated ones, replayed) with digits / on the
-// CUDA cores, ms: 20 lanes, random 4 layers 1.29 (0.61) / 1.13 (0.81), 20 layers 6.28
-// (1.96) / 4.95 (2.92), QFT 1.32 (0.83) / 1.22 (1.13), Ising 1.65 (0.85) / 1.39 (1.29);
-// 21 lanes, 1.66 (0.90) / 1.70 (1.40), 6.30 (2.66) / 7.01 (5.02), 1.69 (1.22) / 2.10 (1.98), 2.01
-// (1.19) / 2.31 (2.21); 23 lanes, 2.74 / 4.47, 9.1 / 18.3, 3.07 / 6.05, 3.35 / 6.34.
+// CUDA cores, ms: 20 lanes, random 4 layers 1.09 (0.60) / 1.13 (0.81), 20 layers 5.22
+// (1.89) / 4.95 (2.89), QFT 1.14 (0.86) / 1.21 (1.11), Ising 1.38 (0.86) / 1.38 (1.28);
+// 21 lanes, 1.42 (0.92) / 1.66 (1.39), 5.13 (2.54) / 6.94 (4.99), 1.46 (1.21) / 2.08 (1.94),
+// 1.72 (1.13) / 2.31 (2.19); 23 lanes, 2.52 / 4.43, 8.8 / 18.1, 3.0 / 6.0, 2.99 / 6.25.
 constexpr int kDigitLanes = 21;
 static bool tensor_stages_pay(const Device &d, const States *s) {
     return d.tensor_blocks &&

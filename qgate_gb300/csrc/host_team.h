@@ -23,10 +23,11 @@ class HostTeam {
 public:
     // Calls f(0), .., f(parts - 1), each once, on up to omp_get_max_threads()
     // threads, the caller's among them; f must not throw.  Called while the helpers
-    // are at work (by another thread, or from within f), it makes all the calls itself.
+    // are at work (by another thread, or from within f) or from an OpenMP region, it
+    // makes all the calls itself.
     template <class F> static void run(int parts, const F &f) {
         std::atomic<bool> &taken = in_run();
-        if (parts > 1 && !taken.exchange(true)) {
+        if (parts > 1 && !omp_in_parallel() && !taken.exchange(true)) {
             HostTeam &t = team();
             const int helpers = t.ready(std::min(parts, omp_get_max_threads()) - 1);
             std::atomic<int> next(0), busy(helpers);

@@ -146,8 +146,10 @@ unsigned long long plan_stage_lanes(const std::vector<const PendingGate *> &rema
     // Multi-start: the plain greedy growth, and growths seeded with each
     // of the few lanes that take the most gates on their own; keep the
     // best.
-    unsigned long long S = grow(fixed);
-    int cur = stage_take(remaining, S, kWindow, nullptr, nullptr);
+    // (The growths run on the host threads: 35 instead of 80 us of Grace for a stage of
+    // 21 lanes, which a circuit that is run once waits for.)
+    unsigned long long S;
+    int cur;
     {
         std::vector<std::pair<int, int>> seeds;
         for (unsigned long long c = cand_all & ~fixed; c; c &= c - 1) {
@@ -156,14 +158,20 @@ unsigned long long plan_stage_lanes(const std::vector<const PendingGate *> &rema
                 -stage_take(remaining, fixed | (1ULL << lane), kWindow, nullptr, nullptr), lane);
         }
         std::sort(seeds.begin(), seeds.end());
-        for (size_t k = 0; k < seeds.size() && k < 6 && __builtin_popcountll(fixed) < M; ++k) {
-            const unsigned long long T = grow(fixed | (1ULL << seeds[k].second));
-            const int got = stage_take(remaining, T, kWindow, nullptr, nullptr);
-            if (got > cur) {
-                S = T;
-                cur = got;
+        const int more = __builtin_popcountll(fixed) < M ? (int)std::min<size_t>(seeds.size(), 6) : 0;
+        unsigned long long grown[7];
+        int got[7];
+        HostTeam::run(1 + more, [&](int k) {
+            grown[k] = grow(k ? fixed | (1ULL << seeds[k - 1].second) : fixed);
+            got[k] = stage_take(remaining, grown[k], kWindow, nullptr, nullptr);
+        });
+        S = grown[0];
+        cur = got[0];
+        for (int k = 1; k <= more; ++k)
+            if (got[k] > cur) {
+                S = grown[k];
+                cur = got[k];
             }
-        }
     }
     // Swap pass: replace a chosen lane (not a low lane or one of the
     // first gate's) by an outside lane while that lets the stage take
