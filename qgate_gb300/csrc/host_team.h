@@ -30,12 +30,17 @@ public:
         if (parts > 1 && !omp_in_parallel() && !taken.exchange(true)) {
             HostTeam &t = team();
             const int helpers = t.ready(std::min(parts, omp_get_max_threads()) - 1);
-            std::atomic<int> next(0), busy(helpers);
-            const Job job = {[](const void *fn, int part) { (*(const F *)fn)(part); }, &f, parts,
-                             &next, &busy};
-            for (int k = 0; k < helpers; ++k) t.workers_[k]->start(&job);
-            job.work();
-            while (busy.load(std::memory_order_acquire) != 0) std::this_thread::yield();
+            Job *job = new Job{[](const void *fn, int part) { (*(const F *)fn)(part); }, &f, parts};
+            for (int k = 0; k < helpers; ++k) {
+                job->refs.fetch_add(1, std::memory_order_relaxed);
+                t.workers_[k]->start(job);
+            }
+            job->work();
+            // helpers that have not come to it (the cores are busy) are not waited for
+            for (int k = 0; k < helpers; ++k)
+                if (Job *left = t.workers_[k]->job.exchange(nullptr)) left->drop();
+            while (job->done.load(std::memory_order_acquire) < parts) std::this_thread::yield();
+            job->drop();
             taken.store(false);
             return;
         }
@@ -43,26 +48,34 @@ public:
     }
 
 private:
+    // A job lives until its last helper has seen it; f is called only while run waits
+    // for the part.
     struct Job {
         void (*call)(const void *, int);
         const void *fn;
         int parts;
-        std::atomic<int> *next, *busy;
-        void work() const {
-            for (int p; (p = next->fetch_add(1, std::memory_order_relaxed)) < parts;) call(fn, p);
+        std::atomic<int> next{0}, done{0}, refs{1};
+        void work() {
+            for (int p; (p = next.fetch_add(1, std::memory_order_relaxed)) < parts;) {
+                call(fn, p);
+                done.fetch_add(1, std::memory_order_release);
+            }
+        }
+        void drop() {
+            if (refs.fetch_sub(1, std::memory_order_acq_rel) == 1) delete this;
         }
     };
     // Looks for its next job for 100 us (pieces often follow one another), then sleeps.
     struct Worker {
         std::mutex m;
         std::condition_variable cv;
-        std::atomic<const Job *> job{nullptr};
+        std::atomic<Job *> job{nullptr};
         std::atomic<bool> asleep{false};
-        void start(const Job *j) {
+        void start(Job *j) {
             job.store(j);
-            if (!asleep.load()) return;  // (it looks for the job after saying that it sleeps)
-            std::lock_guard<std::mutex> lk(m);
-            cv.notify_one();
+            // Not under m: a worker on its way to sleep may miss this one, and run then
+            // takes the job back.
+            if (asleep.load()) cv.notify_one();
         }
         void loop() {
             for (;;) {
@@ -75,9 +88,10 @@ private:
                     cv.wait(lk, [&] { return job.load() != nullptr; });
                     asleep.store(false);
                 }
-                const Job *j = job.exchange(nullptr);
-                j->work();
-                j->busy->fetch_sub(1, std::memory_order_release);  // the job ends with it
+                if (Job *j = job.exchange(nullptr)) {  // (not taken back meanwhile)
+                    j->work();
+                    j->drop();
+                }
             }
         }
     };

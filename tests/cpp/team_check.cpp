@@ -1,7 +1,9 @@
 // CPU check of the host threads (qgate_gb300/csrc/host_team.h), built and run by
 // tests/test_cpu_host_threads.py: every part runs once, for few and many parts,
 // after pauses in which the helpers fall asleep, from several threads at a time,
-// from within a part, and in a forked child.  Prints "ok" or what failed.
+// from within a part, and in a forked child; and a run does not wait for helpers
+// that get no core (other threads spin on them all, as a BLAS's do after a call).
+// Prints "ok" or what failed.
 #include "host_team.h"
 
 #include <sys/wait.h>
@@ -37,6 +39,24 @@ int main() {
     std::atomic<int> inner(0);
     HostTeam::run(6, [&](int) { HostTeam::run(3, [&](int) { inner.fetch_add(1); }); });
     if (inner != 18) return printf("nested: %d\n", inner.load()), 1;
+    std::atomic<bool> stop(false);
+    std::vector<std::thread> spinners;
+    for (int k = 0; k < 2 * (int)std::thread::hardware_concurrency(); ++k)
+        spinners.emplace_back([&] {
+            while (!stop.load(std::memory_order_relaxed)) {
+            }
+        });
+    std::vector<double> us;
+    for (int i = 0; i < 61; ++i) {
+        usleep(300);
+        const auto t = std::chrono::steady_clock::now();
+        if (!once(6)) bad = true;
+        us.push_back(std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t).count());
+    }
+    stop = true;
+    for (auto &t : spinners) t.join();
+    std::sort(us.begin(), us.end());
+    if (bad || us[30] > 1000.) return printf("busy cores: median %.0f us\n", us[30]), 1;
     const pid_t child = fork();
     if (child == 0) _exit(once(9) ? 0 : 1);
     int status = 1;
