@@ -236,8 +236,9 @@ int qg_tensor_stage_raise(int status);
 int qg_gate_stats(int64_t *gates, int64_t *passes, int64_t *bytes, int reset);
 
 /* Extension: per-kernel-class launch timing with CUDA events recorded on the
- * engine's stream around each launch (classes: stage, gate, multi, init,
- * prob, pauli, measure, join, gather, marginal, scan, search, batch). */
+ * engine's stream around each launch (classes: stage, tstage, marked, phase,
+ * gate, multi, init, prob, pauli, measure, join, gather, marginal, scan,
+ * search, batch). */
 int qg_timing_enable(int on);
 int qg_timing_read(const char *kernel_class, int64_t *launches, double *total_ms, int reset);
 /* Extension: device facts {SMs, max opt-in shared memory per block, L2 bytes,

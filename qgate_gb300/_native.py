@@ -224,8 +224,8 @@ def timing_read(kernel_class, reset=False):
     return n.value, ms.value
 
 
-KERNEL_CLASSES = ('stage', 'tstage', 'gate', 'multi', 'init', 'prob', 'pauli', 'measure', 'join',
-                  'gather', 'marginal', 'scan', 'search', 'batch')
+KERNEL_CLASSES = ('stage', 'tstage', 'marked', 'phase', 'gate', 'multi', 'init', 'prob', 'pauli',
+                  'measure', 'join', 'gather', 'marginal', 'scan', 'search', 'batch')
 
 
 def timing_all(reset=False):
